@@ -390,7 +390,8 @@ int tapgpu_set_scenario_links(tapgpu_ctx *ctx, int num_scen, const int64_t *edit
  * (scenario, origin) tasks, out[2] node expansions, and for the near-far
  * kernels out[3] idle polls of warps that found no near work, out[4] warp
  * batches of up to 32 expansions and out[5] (queue variant) nodes claimed by
- * the bitmap word scan instead of the ring. */
+ * the bitmap word scan instead of the ring.  (Label-correction kernels only:
+ * iterations on the elimination hierarchy leave them as they are.) */
 int tapgpu_get_path_stats(tapgpu_ctx *ctx, int64_t *out);
 
 /* No counterpart in the reference.  All-origins FP64 shortest-path labels for

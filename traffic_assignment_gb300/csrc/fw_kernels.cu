@@ -1856,6 +1856,7 @@ constexpr int kLinkBlock = 256;
 // With from_x set, x is taken as given (warm start).
 __global__ void __launch_bounds__(kLinkBlock) k_init_flows(LinkArgs a, int from_x) {
   const int scen = scen_of(a);
+  if (a.state[scen].done > 1) return;  // paused in its first loading: nothing to start from
   const size_t off = static_cast<size_t>(scen) * a.m;
   const double* cap = a.cap + off;
   for (int k = blockIdx.x * kLinkBlock + threadIdx.x; k < a.m; k += gridDim.x * kLinkBlock) {
@@ -1905,6 +1906,14 @@ __global__ void __launch_bounds__(kLinkBlock) k_set_free_flow(LinkArgs a) {
     a.y_fx[off + k] = 0ull;
     write_weights(a, scen, k, a.lp.fft[lpi(a.lp, scen, k)]);
   }
+}
+
+// the records of every link at its current cost
+__global__ void __launch_bounds__(kLinkBlock) k_records(LinkArgs a) {
+  const int scen = scen_of(a);
+  const size_t off = static_cast<size_t>(scen) * a.m;
+  for (int k = blockIdx.x * kLinkBlock + threadIdx.x; k < a.m; k += gridDim.x * kLinkBlock)
+    write_weights(a, scen, k, a.t[off + k]);
 }
 
 // candidate step j of a pass: 2^-(e0+j) (reference rule) or the j-th of 12
@@ -2503,6 +2512,11 @@ cudaError_t launch_init_flows(const LinkArgs& a, int grid, cudaStream_t s) {
 
 cudaError_t launch_set_costs(const LinkArgs& a, int grid, cudaStream_t s) {
   k_set_free_flow<<<dim3(grid, a.num_scen), kLinkBlock, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_records(const LinkArgs& a, int grid, cudaStream_t s) {
+  k_records<<<dim3(grid, a.num_scen), kLinkBlock, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -51,11 +51,12 @@ struct LinkParams {
 
 struct ScenState {
   int iter;        // FW iterations completed
-  int done;        // 1 once the stopping rule holds
+  int done;        // 1 once the stopping rule holds (above 1: paused, see hier_kernels.cuh)
   int ls_pending;  // line search still searching
   int ls_next;     // next halving exponent to test
   int max_iters;   // <= 0: no cap
-  int pad0, pad1, pad2;
+  int u_exp;       // integer path labels: costs are scaled by 2^u_exp
+  unsigned long long maxlab;  // largest integer label of the iteration
   double target_relgap;
   double relgap, best_lb, obj, gap, lambda, vht, avg_excess, g0;
   double vht_end;  // VHT at the current x with the current costs
@@ -199,6 +200,8 @@ cudaError_t launch_set_costs(const LinkArgs& a, int grid, cudaStream_t s);
 // line-search passes and the step: `block` kSmallLinkBlock (networks of at
 // most kSmallNet links, FP64 work over more SMs) or kLinkBlock
 constexpr int kSmallLinkBlock = 64;
+// weights of the label-correction kernels' records from the current costs t
+cudaError_t launch_records(const LinkArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_ls_pass(const LinkArgs& a, int grid, int block, cudaStream_t s);
 cudaError_t launch_ls_fallback(const LinkArgs& a, cudaStream_t s);
 cudaError_t launch_step(const LinkArgs& a, int grid, int block, cudaStream_t s);

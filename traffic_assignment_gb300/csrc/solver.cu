@@ -8,9 +8,12 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <memory>
+#include <functional>
 #include <limits>
+#include <memory>
 #include <numeric>
+#include <system_error>
+#include <thread>
 
 namespace tapgpu {
 
@@ -190,7 +193,7 @@ PathArgs Ctx::path_args(int nscen_slots) const {
   a.all_global = opt.global_scratch == 2;
   a.stats = timing ? path_stats : nullptr;
   a.nf_delta = nf_delta;
-  a.e4 = (!fp64 && (sssp_variant == kSsspNearFarQueue || sssp_variant == kSsspNearFarQueueWide))
+  a.e4 = (!fp64 && e4 && (sssp_variant == kSsspNearFarQueue || sssp_variant == kSsspNearFarQueueWide))
              ? e4
              : nullptr;
   a.r4 = rev4 ? r4 : nullptr;
@@ -200,7 +203,7 @@ PathArgs Ctx::path_args(int nscen_slots) const {
   return a;
 }
 
-LinkArgs Ctx::link_args(int nscen) const {
+LinkArgs Ctx::link_args(int nscen, bool records) const {
   LinkArgs a;
   std::memset(&a, 0, sizeof(a));
   a.m = M;
@@ -212,20 +215,27 @@ LinkArgs Ctx::link_args(int nscen) const {
   a.t = t;
   a.d = d;
   a.y_fx = yfx;
-  a.e32 = fp64 ? nullptr : e32;
-  a.r32 = fp64 ? nullptr : r32;
-  a.e4 = fp64 ? nullptr : e4;
+  // the label-correction kernels' records (with the hierarchy only where
+  // those kernels take over)
+  records |= !hier_on;
+  if (records && !fp64) {
+    a.e32 = e32;
+    a.r32 = r32;
+    a.e4 = e4;
+    a.r4 = rev4 ? r4 : nullptr;
+  }
+  if (records && fp64) {
+    a.r4d = r4d;
+    a.w64 = w64;
+  }
   a.ell_pos = ell_pos;
   a.e4x = e4x;
-  a.r4 = rev4 && !fp64 ? r4 : nullptr;
-  a.r4d = fp64 ? r4d : nullptr;
   a.r4_pos = r4_pos;
   a.r4x = r4x;
   a.n1 = n1;
   a.head = head;
   a.tail = tail;
   a.rpos = rpos;
-  a.w64 = fp64 ? w64 : nullptr;
   a.dtdx = dtdx;
   a.partials = partials;
   a.arrive = arrive;
@@ -274,6 +284,82 @@ int Ctx::ensure_scenarios(int S) {
   TG_TRY(alloc_n(&t, sm));
   TG_TRY(alloc_n(&d, sm));
   TG_TRY(alloc_n(&yfx, sm));
+  S_cap = S;
+  if (opt.record_tape) TG_TRY(alloc_n(&dtdx, sm));
+  TG_TRY(alloc_n(&state, static_cast<size_t>(S)));
+  TG_TRY(alloc_n(&partials, static_cast<size_t>(S) * std::max(link_grid, ls_link_grid) * kNumSums));
+  TG_TRY(alloc_n(&arrive, static_cast<size_t>(S)));
+  TG_CUDA(cudaMemset(arrive, 0, sizeof(unsigned) * S));
+  trace_cap = S == 1 ? 100000 : 4096;
+  TG_TRY(alloc_n(&trace, static_cast<size_t>(S) * trace_cap * kTraceCols));
+  TG_TRY(alloc_n(&scen_list, static_cast<size_t>(S)));
+  h_scen_list.clear();
+  if (opt.record_tape && opt.tape_capacity > 0) {
+    hist_cap = opt.tape_capacity;
+    ckpt_every = opt.tape_checkpoint > 0
+                     ? opt.tape_checkpoint
+                     : std::max(1, static_cast<int>(std::ceil(std::sqrt(double(hist_cap)))));
+    TG_TRY(alloc_n(&x_hist, sm * (hist_cap / ckpt_every + 1)));
+    TG_TRY(alloc_n(&d_hist, sm * hist_cap));
+    TG_TRY(alloc_n(&lam_hist, static_cast<size_t>(S) * hist_cap));
+  }
+  if (gexec) {
+    cudaGraphExecDestroy(gexec);
+    gexec = nullptr;
+  }
+  g_nscen = -1;
+  return TAPGPU_OK;
+}
+
+// Whether an iteration of nscen scenarios takes less time on the hierarchy than
+// on the label-correction kernels.  Both times (us) from fits to measurements
+// on synthetic city networks of 1,200 to 40,000 nodes, 40 to 1,000 origins and 1
+// to 64 scenarios, FP64:
+//   label correction: one task 100 + 27 n/1000 or 250 + 15.5 n/1000 (80 n/1000
+//     with its labels in global memory); among many, 0.05 + 0.132 n/1000 each
+//     (0.17 where one of them fills an SM)
+//   hierarchy: its levels one after the other, 140 + 25 each, however little
+//     there is to do; 3.5 per 10^6 relaxations of an elimination per
+//     scenario; 1.2 per 10^6 arcs and origin
+// Measured, hierarchy : label correction in ms: 10,000 nodes, 1,000 origins, 1
+// scenario 1.34 : 1.70, 4 scenarios 2.31 : 5.77, 16 scenarios 6.04 : 22.2; 40
+// origins, 64 scenarios 5.42 : 3.66; 3,569 nodes, 101 origins, 16 scenarios
+// 1.08 : 0.93, 64 scenarios 1.93 : 3.14; 22,500 nodes, 400 origins, 1 scenario
+// 2.02 : 1.86, 2 scenarios 2.24 : 3.55.
+bool Ctx::hier_pays(int nscen, int levels, double relaxations, int arcs) const {
+  const double kn = n1 * 1e-3, tasks = static_cast<double>(nscen) * Z;
+  const double one = sssp_smem ? std::min(100.0 + 27.0 * kn, 250.0 + 15.5 * kn) : 80.0 * kn;
+  const double each = 0.05 + (sssp_smem && sssp_grid <= num_sms ? 0.17 : 0.132) * kn;
+  const double corrected = std::max(one, 0.75 * one + each * tasks);
+  const double swept = 140.0 + 25.0 * levels + 3.5e-6 * relaxations * nscen + 1.2e-6 * arcs * tasks;
+  return corrected > 1.05 * swept;
+}
+
+// The path kernels of the next iterations of nscen scenarios, and their buffers.
+int Ctx::choose_paths(int nscen) {
+  bool on = hier && hier_pays(nscen, static_cast<int>(h_tile_ptr.size()) - 1, hier_relaxations, hg.arcs);
+  if (on && hier_cap < nscen) {
+    if (gexec) cudaGraphExecDestroy(gexec);
+    gexec = nullptr;
+    if (ensure_hier(nscen) != TAPGPU_OK) {  // no room: the label-correction kernels
+      cudaGetLastError();
+      release_hier();
+      on = false;
+    }
+  }
+  if (!on) TG_TRY(ensure_legacy(S_cap));
+  if (on != hier_on && gexec) {
+    cudaGraphExecDestroy(gexec);
+    gexec = nullptr;
+  }
+  hier_on = on;
+  return TAPGPU_OK;
+}
+
+// The weight records and the label buffer of the label-correction kernels.
+int Ctx::ensure_legacy(int S) {
+  if (fp64 ? w64 != nullptr : e32 != nullptr) return TAPGPU_OK;
+  const size_t sm = static_cast<size_t>(S) * M;
   if (fp64) {
     TG_TRY(alloc_n(&w64, sm));
     // slots beyond a node's in-links keep an infinite weight: never tight
@@ -293,24 +379,6 @@ int Ctx::ensure_scenarios(int S) {
       TG_CUDA(launch_fill_records(r4, s4, make_uint2(0u, 0x7f800000u), 2 * num_sms, stream));
     }
   }
-  if (opt.record_tape) TG_TRY(alloc_n(&dtdx, sm));
-  TG_TRY(alloc_n(&state, static_cast<size_t>(S)));
-  TG_TRY(alloc_n(&partials, static_cast<size_t>(S) * std::max(link_grid, ls_link_grid) * kNumSums));
-  TG_TRY(alloc_n(&arrive, static_cast<size_t>(S)));
-  TG_CUDA(cudaMemset(arrive, 0, sizeof(unsigned) * S));
-  trace_cap = S == 1 ? 100000 : 4096;
-  TG_TRY(alloc_n(&trace, static_cast<size_t>(S) * trace_cap * kTraceCols));
-  TG_TRY(alloc_n(&scen_list, static_cast<size_t>(S)));
-  if (opt.record_tape && opt.tape_capacity > 0) {
-    hist_cap = opt.tape_capacity;
-    ckpt_every = opt.tape_checkpoint > 0
-                     ? opt.tape_checkpoint
-                     : std::max(1, static_cast<int>(std::ceil(std::sqrt(double(hist_cap)))));
-    TG_TRY(alloc_n(&x_hist, sm * (hist_cap / ckpt_every + 1)));
-    TG_TRY(alloc_n(&d_hist, sm * hist_cap));
-    TG_TRY(alloc_n(&lam_hist, static_cast<size_t>(S) * hist_cap));
-  }
-  S_cap = S;
   // Unless the caller fixed the chunk, the label buffer grows to hold a whole
   // batch's tasks (up to 16 GiB), so that an iteration runs one shortest-path
   // and one loading launch instead of one per chunk, each with its tail.
@@ -329,11 +397,352 @@ int Ctx::ensure_scenarios(int S) {
       }
     }
   }
-  if (gexec) {
-    cudaGraphExecDestroy(gexec);
-    gexec = nullptr;
+  return TAPGPU_OK;
+}
+
+// ---------------------------------------------------------------------------
+// elimination hierarchy
+// ---------------------------------------------------------------------------
+
+// The host plan, made by a thread of its own while the context is set up
+// (10,000 nodes: 9 of the 13 ms that the hierarchy adds to the setup).
+class HierBuilder {
+ public:
+  // the network in link order; dem: the caller's demand (origins 1..Z)
+  HierBuilder(const Ctx& c, const tapgpu_demand* dem) {
+    if (!wanted(c)) return;
+    auto work = [this, &c, dem] {
+      try {
+        std::vector<char> dests(c.n1, 0);
+        for (int o = 1; dem && o <= c.Z; ++o)
+          for (int64_t i = dem->od_ptr[o]; i < dem->od_ptr[o + 1]; ++i) {
+            const int64_t d = dem->od_dest[i];
+            if (d < 0 || d >= c.n1) return;  // (reported when it is loaded)
+            if (dem->od_demand[i] > 0 && d != o) dests[d] = 1;
+          }
+        built_ = hier_build(c.n1, c.M, c.h_tail.data(), c.h_head.data(), c.F, dests, 80.0 * c.n1,
+                            1e11, plan_);
+      } catch (const std::bad_alloc&) {
+      }
+    };
+    try {
+      thread_ = std::thread(work);
+    } catch (const std::system_error&) {
+      work();
+    }
   }
-  g_nscen = -1;
+  ~HierBuilder() { wait(); }
+  const HierPlan* wait() {
+    if (thread_.joinable()) thread_.join();
+    return built_ ? &plan_ : nullptr;
+  }
+
+ private:
+  // FP64 paths (integer labels break near-ties as exact sums do, which FP64
+  // sums do too; the FP32 sums' ties fall otherwise).  A caller's choice of a
+  // label-correction kernel or of its shape stands; networks small enough for
+  // the edge-list sweeps keep them.
+  static bool wanted(const Ctx& c) {
+    const tapgpu_options& o = c.opt;
+    return c.fp64 && c.Z >= 1 && (c.n1 > kSmallNet || c.M > kSmallNet) &&
+           !(o.sssp_variant || o.sssp_block || o.aon_block || o.nf_delta > 0 || o.global_scratch ||
+             o.chunk_tasks || o.sssp_ctas_per_sm || o.aon_ctas_per_sm);
+  }
+
+  HierPlan plan_;
+  bool built_ = false;
+  std::thread thread_;
+};
+
+// The plan on the device, where the hierarchy can pay.  (odest, optr, odem: the
+// demand as a CSR over origin slots)
+int Ctx::hier_plan(const HierPlan* plan, const std::vector<int>& odest, const std::vector<int>& optr,
+                   const std::vector<double>& odem) {
+  hier = false;
+  if (!plan) return TAPGPU_OK;
+  const HierPlan& p = *plan;
+  if (hier_climb_smem(p.climb) > kHierMaxClimb || p.climb > 0xffff) return TAPGPU_OK;
+  if (!hier_pays(4096, p.num_levels, p.relaxations, p.arcs)) return TAPGPU_OK;
+  std::vector<int> odpos(odest.size(), -1);
+  for (int o = 0; o < Z; ++o)
+    for (int i = optr[o]; i < optr[o + 1]; ++i)
+      if (odem[i] > 0 && odest[i] != o + 1) odpos[i] = odest[i];
+  std::vector<int> dest_of(n1, -1);
+  for (size_t i = 0; i < p.dest_node.size(); ++i) dest_of[p.dest_node[i]] = static_cast<int>(i);
+  for (auto& x : odpos)
+    if (x >= 0) x = dest_of[x];
+
+  hier_relaxations = p.relaxations;
+  hg.n = p.n;
+  hg.arcs = p.arcs;
+  hg.climb = p.climb;
+  hg.num_elims = static_cast<int>(p.elims.size());
+  hg.num_marks = static_cast<int>(p.marks.size());
+  h_tile_ptr = p.tile_ptr;
+  hg.top_rows = p.top_rows;
+  hg.top_levels = p.top_levels;
+  hg.num_subs = static_cast<int>(p.subs.size());
+  std::vector<unsigned short> iclimb(p.idx.size()), aclimb(static_cast<size_t>(p.arcs), 0);
+  for (size_t i = 0; i < p.idx.size(); ++i) {
+    const HierChunk& c = p.chunks[p.chunk_of[p.idx[i]]];
+    iclimb[i] = static_cast<unsigned short>(c.coff + p.idx[i] - c.first);
+  }
+  for (const auto& c : p.chunks)
+    for (int i = 0; i < c.k; ++i)
+      std::fill_n(aclimb.begin() + c.woff + i * c.ld, c.ld, static_cast<unsigned short>(c.coff + i));
+  // one allocation and one copy for all of it
+  std::vector<unsigned char> blob;
+  std::vector<std::function<void(unsigned char*)>> at;
+  auto put = [&](auto** dst, const auto& v) {
+    at.push_back([dst, off = blob.size()](unsigned char* base) {
+      *dst = reinterpret_cast<typename std::remove_reference<decltype(*dst)>::type>(base + off);
+    });
+    const auto* q = reinterpret_cast<const unsigned char*>(v.data());
+    blob.insert(blob.end(), q, q + v.size() * sizeof(v[0]));
+    blob.resize((blob.size() + 255) / 256 * 256);
+  };
+  blob.reserve(sizeof(int) * (8 * static_cast<size_t>(p.arcs) + 8 * p.idx.size() + p.rel.size() +
+                              64 * static_cast<size_t>(n1)));
+  put(&hg.chunks, p.chunks);
+  put(&hg.shut, p.shut);
+  put(&hg.idx, p.idx);
+  put(&hg.idx_climb, iclimb);
+  put(&hg.arc_climb, aclimb);
+  put(&hg.tgt_base, p.tgt_base);
+  put(&hg.tgt_rel, p.tgt_rel);
+  put(&hg.rel, p.rel);
+  put(&hg.arc_link, p.arc_link);
+  put(&hg.link_arc, p.link_arc);
+  put(&hg.link_next, p.link_next);
+  put(&hg.elims, p.elims);
+  put(&hg.elim_pair, p.elim_pair);
+  put(&hg.elim_close, p.elim_close);
+  HierPlan::Node* nodes = nullptr;
+  int* chunk_of = nullptr;
+  put(&nodes, p.nodes);
+  put(&chunk_of, p.chunk_of);
+  put(&hg.tiles, p.tiles);
+  put(&hg.marks, p.marks);
+  put(&hg.tops, p.tops);
+  put(&hg.top_uidx, p.top_uidx);
+  put(&hg.top_dest, p.top_dest);
+  put(&hg.job_ptr, p.job_ptr);
+  put(&hg.jobs, p.jobs);
+  put(&hg.subs, p.subs);
+  put(&hg.sub_ext, p.sub_ext);
+  put(&hg.sub_rows, p.sub_rows);
+  put(&hg.sub_slot, p.sub_slot);
+  put(&hg.sub_ids, p.sub_ids);
+  put(&h_od_dest, odpos);
+  // origins in position order: neighbours in the network share a group
+  std::vector<int> opos(Z), by_pos(Z), column(Z), chain_ptr(Z + 1, 0), chain;
+  for (int o = 0; o < Z; ++o) opos[o] = p.pos[o + 1];
+  std::iota(by_pos.begin(), by_pos.end(), 0);
+  std::sort(by_pos.begin(), by_pos.end(), [&](int a, int b) { return opos[a] < opos[b]; });
+  for (int i = 0; i < Z; ++i) column[by_pos[i]] = i;
+  for (int o = 0; o < Z; ++o) {
+    for (int c = p.chunk_of[opos[o]]; c >= 0; c = p.chunks[c].parent) chain.push_back(c);
+    chain_ptr[o + 1] = static_cast<int>(chain.size());
+  }
+  while (by_pos.size() % kHierWidth) by_pos.push_back(-1);
+  put(&h_opos, opos);
+  put(&h_group, by_pos);
+  put(&h_column, column);
+  put(&h_chain_ptr, chain_ptr);
+  put(&h_chain, chain);
+  unsigned char* dev = nullptr;
+  HierPlan::Pair* pairs = nullptr;
+  TG_TRY(alloc_n(&dev, blob.size()));
+  TG_TRY(alloc_n(&pairs, static_cast<size_t>(p.num_pairs)));
+  TG_CUDA(cudaMemcpyAsync(dev, blob.data(), blob.size(), cudaMemcpyHostToDevice, stream));
+  for (const auto& f : at) f(dev);
+  hg.pairs = pairs;
+  TG_CUDA(launch_hier_pairs(hg, nodes, static_cast<int>(p.nodes.size()), chunk_of, pairs, stream));
+  h_dests = static_cast<int>(p.dest_node.size());
+  h_width = static_cast<int>(by_pos.size());
+  TG_TRY(hier_demand(od_q, 1, &h_dem));
+  // first exponent: twice the largest cost of a path with the fewest links
+  // from the first origin at free flow just fits
+  {
+    std::vector<int> rp(n1 + 1, 0), queue{1};
+    for (int k = 0; k < M; ++k) ++rp[h_tail[k] + 1];
+    for (int v = 0; v < n1; ++v) rp[v + 1] += rp[v];
+    std::vector<double> far(n1, -1.0);
+    far[1] = 0.0;
+    double most = 0.0;
+    for (size_t i = 0; i < queue.size(); ++i) {
+      const int v = queue[i];
+      most = std::max(most, far[v]);
+      for (int k = rp[v]; k < rp[v + 1]; ++k)
+        if (far[h_head[k]] < 0) {
+          far[h_head[k]] = far[v] + h_fft[k];
+          queue.push_back(h_head[k]);
+        }
+    }
+    int e = 0;
+    if (most > 0) e = 59 - static_cast<int>(std::ceil(std::log2(most))) - 1;
+    u_exp0 = std::max(-900, std::min(900, e));
+  }
+  hier = true;
+  return TAPGPU_OK;
+}
+
+// Demand by destination from the OD entries dev_q [nscen][nnz] (device).
+int Ctx::hier_demand(const long long* dev_q, int nscen, unsigned long long** dem) {
+  const size_t row = static_cast<size_t>(h_dests) * h_width;
+  if (!*dem) TG_TRY(alloc_n(dem, row * nscen));
+  TG_CUDA(cudaMemsetAsync(*dem, 0, sizeof(unsigned long long) * row * nscen, stream));
+  TG_CUDA(launch_hier_demand(od_ptr, h_od_dest, dev_q, nnz, nscen, Z, h_column, *dem, h_width,
+                             static_cast<long long>(row), dem != &h_dem, stream));
+  TG_CUDA(cudaStreamSynchronize(stream));
+  return TAPGPU_OK;
+}
+
+void Ctx::release_hier() {
+  void* olds[] = {h_w, h_mid, h_flow, h_d0, h_from, h_via, h_fup, h_dlab, h_vol, h_arr, h_list, h_list_n};
+  for (void* p : olds) free_owned(this, p);
+  h_w = h_mid = h_flow = h_d0 = h_fup = h_dlab = h_vol = nullptr;
+  h_from = h_list = h_list_n = nullptr;
+  h_arr = nullptr;
+  h_via = nullptr;
+  hier_cap = 0;
+}
+
+int Ctx::ensure_hier(int S) {
+  release_hier();
+  const size_t arcs3 = 3 * static_cast<size_t>(hg.arcs);
+  const size_t climb = static_cast<size_t>(Z) * hg.climb;
+  // labels of the top rows for every origin (padded to whole groups)
+  const size_t top = static_cast<size_t>(h_width) * hg.top_rows;
+  // at most 24 GiB of per-scenario buffers; more scenarios take turns in them
+  const size_t per = arcs3 * 32 + climb * 21 + top * 18;
+  hier_slots = static_cast<int>(std::max<size_t>(1, std::min<size_t>(S, (size_t(24) << 30) / per)));
+  const size_t ns = static_cast<size_t>(hier_slots), nc = ns * top;
+  TG_TRY(alloc_n(&h_w, ns * arcs3));
+  TG_TRY(alloc_n(&h_mid, ns * arcs3));
+  TG_TRY(alloc_n(&h_flow, ns * arcs3));
+  TG_TRY(alloc_n(&h_d0, ns * climb));
+  TG_TRY(alloc_n(&h_from, ns * climb));
+  TG_TRY(alloc_n(&h_via, ns * climb));
+  TG_TRY(alloc_n(&h_fup, ns * climb));
+  TG_TRY(alloc_n(&h_dlab, nc));
+  TG_TRY(alloc_n(&h_vol, nc));
+  TG_TRY(alloc_n(&h_arr, nc));
+  TG_TRY(alloc_n(&h_list, ns * 2 * arcs3));
+  TG_TRY(alloc_n(&h_list_n, ns * 4));
+  // volumes are zero between tasks and iterations; padding reads labels of
+  // other rows, which only have to be in range
+  TG_CUDA(cudaMemsetAsync(h_flow, 0, ns * arcs3 * sizeof(unsigned long long), stream));
+  TG_CUDA(cudaMemsetAsync(h_list_n, 0, ns * 4 * sizeof(int), stream));
+  TG_CUDA(cudaMemsetAsync(h_vol, 0, nc * sizeof(*h_vol), stream));
+  TG_CUDA(cudaMemsetAsync(h_dlab, 0, nc * sizeof(*h_dlab), stream));
+  hier_cap = S;
+  return TAPGPU_OK;
+}
+
+// Shortest paths and loading of the first nscen entries of scen_list at link
+// costs cost[scenario * stride + link], into yfx.
+int Ctx::enqueue_hier(int nscen, const double* cost, long long stride, cudaEvent_t between) {
+  HierArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.h = hg;
+  a.m = M;
+  a.num_sources = Z;
+  a.scen_list = scen_list;
+  a.state = state;
+  a.cost = cost;
+  a.cost_stride = stride;
+  a.absent = use_link_scen ? sc_absent : nullptr;
+  a.absent_words = absent_words;
+  a.w = h_w;
+  a.mid = h_mid;
+  a.flow = h_flow;
+  a.d0 = h_d0;
+  a.from = h_from;
+  a.via = h_via;
+  a.fup = h_fup;
+  a.opos = h_opos;
+  a.chain_ptr = h_chain_ptr;
+  a.chain = h_chain;
+  a.dest_dem = use_dem_scen ? h_sc_dem : h_dem;
+  a.dest_stride = use_dem_scen ? static_cast<long long>(h_dests) * h_width : 0;
+  a.dest_width = h_width;
+  a.dlab = h_dlab;
+  a.vol = h_vol;
+  a.arr = h_arr;
+  a.group = h_group;
+  a.groups = h_width / kHierWidth;
+  a.list = h_list;
+  a.list_n = h_list_n;
+  a.y_fx = yfx;
+  for (int s0 = 0; s0 < nscen; s0 += hier_slots) {
+    a.slot0 = s0;
+    a.nslots = std::min(hier_slots, nscen - s0);
+    if (measuring) TG_TRY(mark(0, true));
+    const int levels = static_cast<int>(h_tile_ptr.size()) - 1;
+    TG_CUDA(launch_hier_eliminate(a, levels, h_tile_ptr.data(), stream));
+    TG_CUDA(launch_hier_climb(a, stream));
+    TG_CUDA(launch_hier_sweep(a, num_sms, stream));
+    if (measuring) TG_TRY(mark(0, false));
+    if (between) TG_CUDA(cudaEventRecord(between, stream));
+    if (measuring) TG_TRY(mark(1, true));
+    TG_CUDA(launch_hier_load(a, num_sms, stream));
+    if (measuring) TG_TRY(mark(1, false));
+    count_launches(levels + 24);
+  }
+  return TAPGPU_OK;
+}
+
+// Scenarios that left the integers' range repeat their iteration at a smaller
+// exponent (those that used too little of it have their new one); one that
+// does so repeatedly takes this iteration with the label-correction kernels,
+// which also report a missing path.
+constexpr int kHierRetries = 4;
+constexpr int kHierRetryBits = 5;
+
+int Ctx::resume_paused(int S, std::vector<ScenState>& st) {
+  if (!hier_on) return TAPGPU_OK;
+  std::vector<int> legacy;
+  bool any = false;
+  hier_retry.resize(S, {-1, 0});
+  for (int s = 0; s < S; ++s) {
+    if (st[s].done <= 1) continue;
+    any = true;
+    const bool coarse = st[s].done == kCoarse;  // (its exponent is set)
+    auto& r = hier_retry[s];
+    if (r.first != st[s].iter) r = {st[s].iter, 0};
+    st[s].done = 0;
+    st[s].maxlab = 0;
+    if (++r.second > kHierRetries)
+      legacy.push_back(s);
+    else if (!coarse)
+      st[s].u_exp -= kHierRetryBits;
+    TG_CUDA(cudaMemcpyAsync(state + s, &st[s], sizeof(ScenState), cudaMemcpyHostToDevice, stream));
+  }
+  if (!any) return TAPGPU_OK;
+  // a paused scenario's volumes stayed where they were
+  TG_CUDA(cudaMemsetAsync(h_flow, 0,
+                          static_cast<size_t>(hier_slots) * 3 * hg.arcs * sizeof(unsigned long long),
+                          stream));
+  TG_CUDA(cudaStreamSynchronize(stream));
+  if (legacy.empty()) return TAPGPU_OK;
+  TG_TRY(ensure_legacy(S_cap));
+  TG_TRY(set_active(legacy));
+  const int n = static_cast<int>(legacy.size());
+  LinkArgs la = link_args(n, true);
+  TG_CUDA(cudaMemsetAsync(yfx, 0, sizeof(unsigned long long) * static_cast<size_t>(S_cap) * M, stream));
+  TG_CUDA(launch_records(la, link_grid, stream));
+  TG_TRY(enqueue_paths(n, true, e32, r32, w64, yfx, true));
+  TG_TRY(enqueue_tail(n));
+  TG_TRY(sync_check());
+  return read_states(S, st);
+}
+
+int Ctx::set_active(const std::vector<int>& active) {
+  if (active == h_scen_list) return TAPGPU_OK;
+  h_scen_list = active;
+  TG_CUDA(cudaMemcpyAsync(scen_list, h_scen_list.data(), sizeof(int) * active.size(),
+                          cudaMemcpyHostToDevice, stream));
   return TAPGPU_OK;
 }
 
@@ -406,7 +815,8 @@ int Ctx::enqueue_paths(int nscen, bool load, const uint2* e32p, const uint2* r32
   for (int64_t t0 = 0; t0 < tasks; t0 += dist_tasks) {
     const int64_t t1 = std::min(tasks, t0 + dist_tasks);
     PathArgs a = path_args(nscen);
-    if (a.e4) a.e4 = e32p == e32 ? e4 : (e32p == api_e32 ? api_e4 : nullptr);
+    if (!fp64 && (sssp_variant == kSsspNearFarQueue || sssp_variant == kSsspNearFarQueueWide))
+      a.e4 = e32p == api_e32 ? api_e4 : e4;
     a.e32 = e32p;
     a.r32 = r32p;
     if (r32p != r32) a.r4 = nullptr;  // (the padded reverse records follow the context's own)
@@ -451,9 +861,15 @@ void Ctx::count_launches(long long n) {
 
 int Ctx::enqueue_iteration(int nscen) {
   measuring = true;
-  int rc = enqueue_paths(nscen, true, e32, r32, w64, yfx, true);
+  const int rc = hier_on ? enqueue_hier(nscen, t, M)
+                      : enqueue_paths(nscen, true, e32, r32, w64, yfx, true);
   measuring = false;
   TG_TRY(rc);
+  return enqueue_tail(nscen);
+}
+
+// line search and step of an iteration
+int Ctx::enqueue_tail(int nscen) {
   LinkArgs la = link_args(nscen);
   if (M <= kSmallTail) {  // small networks: the line search and the step in one launch
     TG_TRY(mark(2, true));
@@ -479,18 +895,42 @@ int Ctx::enqueue_iteration(int nscen) {
 
 // State reset, first all-or-nothing at free-flow costs (or warm flows), costs.
 int Ctx::enqueue_initial(int nscen, bool warm) {
+  if (!warm) TG_TRY(begin_paths(nscen));
   LinkArgs la = link_args(nscen);
-  if (!warm) {
-    TG_CUDA(launch_set_costs(la, link_grid, stream));
-    count_launches(1);
-    TG_TRY(enqueue_paths(nscen, true, e32, r32, w64, yfx, true));
-    la.pass = 0;
-  } else {
-    la.pass = 1;
-  }
+  la.pass = warm ? 1 : 0;
   TG_CUDA(launch_init_flows(la, link_grid, stream));
   count_launches(1);
   return TAPGPU_OK;
+}
+
+// All-or-nothing at free-flow costs of the first nscen entries of scen_list
+int Ctx::begin_paths(int nscen) {
+  if (hier_on) {
+    const LinkParams lp = link_params();
+    std::vector<ScenState> st;
+    for (int tries = 0; tries <= kHierRetries; ++tries) {
+      TG_TRY(enqueue_hier(nscen, lp.fft, lp.stride));
+      TG_TRY(read_states(nscen, st));
+      bool paused = false;
+      for (int s = 0; s < nscen; ++s) {
+        if (st[s].done <= 1) continue;
+        paused = true;
+        if (st[s].done == kPaused) st[s].u_exp -= kHierRetryBits;
+        st[s].done = 0;
+        st[s].maxlab = 0;
+        TG_CUDA(cudaMemcpyAsync(state + s, &st[s], sizeof(ScenState), cudaMemcpyHostToDevice,
+                                stream));
+      }
+      if (!paused) return TAPGPU_OK;
+      TG_CUDA(cudaMemsetAsync(h_flow, 0, static_cast<size_t>(hier_slots) * 3 * hg.arcs *
+                                             sizeof(unsigned long long), stream));
+      TG_CUDA(cudaStreamSynchronize(stream));
+    }
+    TG_TRY(ensure_legacy(S_cap));  // (which also reports a missing path)
+  }
+  TG_CUDA(launch_set_costs(link_args(nscen, true), link_grid, stream));
+  count_launches(1);
+  return enqueue_paths(nscen, true, e32, r32, w64, yfx, true);
 }
 
 int Ctx::run_graph(int iters, int nscen) {
@@ -696,6 +1136,8 @@ static int create_impl(const tapgpu_network* net, const tapgpu_demand* dem,
     c->nf_delta = opt.nf_delta > 0 ? opt.nf_delta : (mean > 0 ? 16.0 * mean : 1.0);
   }
 
+  HierBuilder builder(*c, dem);
+
   std::vector<int> rp(n1 + 1, 0), ip_in(n1 + 1, 0), inl(M);
   for (int k = 0; k < M; ++k) {
     rp[c->h_tail[k] + 1]++;
@@ -837,6 +1279,7 @@ static int create_impl(const tapgpu_network* net, const tapgpu_demand* dem,
 
   TG_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   TG_TRY(c->plan_launches());
+  TG_TRY(c->hier_plan(builder.wait(), odest, optr, odem));
   TG_TRY(c->alloc_n(&c->counters, 2));
   TG_TRY(c->alloc_n(&c->err, 1));
   TG_TRY(c->alloc_n(&c->err_info, 2));
@@ -857,6 +1300,7 @@ static int create_impl(const tapgpu_network* net, const tapgpu_demand* dem,
   TG_TRY(c->alloc_n(&c->api_w64, M));
   TG_TRY(c->alloc_n(&c->api_yfx, M));
   TG_TRY(c->ensure_scenarios(1));
+  TG_TRY(c->choose_paths(1));
   std::vector<double> capv(c->h_cap);
   TG_CUDA(cudaMemcpy(c->cap, capv.data(), sizeof(double) * M, cudaMemcpyHostToDevice));
   *out = guard.release();
@@ -871,7 +1315,9 @@ static int upload_states(Ctx* c, int S, int max_iters, double target) {
     s.target_relgap = target;
     s.relgap = DBL_MAX;
     s.best_lb = -DBL_MAX;
+    s.u_exp = c->u_exp0;
   }
+  c->hier_retry.clear();
   TG_CUDA(cudaMemcpyAsync(c->state, st.data(), sizeof(ScenState) * S, cudaMemcpyHostToDevice,
                           c->stream));
   TG_CUDA(cudaMemsetAsync(c->err, 0, sizeof(int), c->stream));
@@ -885,10 +1331,11 @@ static int iterate_until_done(Ctx* c, int S, int max_iters, std::vector<ScenStat
   std::vector<int> active;
   for (;;) {
     TG_TRY(c->read_states(S, st));
+    TG_TRY(c->sync_check());
+    TG_TRY(c->resume_paused(S, st));
     active.clear();
     for (int s = 0; s < S; ++s)
       if (!st[s].done) active.push_back(s);
-    TG_TRY(c->sync_check());
     if (active.empty()) break;
     int n = per;
     if (max_iters > 0) {
@@ -896,11 +1343,7 @@ static int iterate_until_done(Ctx* c, int S, int max_iters, std::vector<ScenStat
       for (int s : active) left = std::max(left, max_iters - st[s].iter);
       n = std::max(1, std::min(n, left));
     }
-    if (active != c->h_scen_list) {
-      TG_CUDA(cudaMemcpyAsync(c->scen_list, active.data(), sizeof(int) * active.size(),
-                              cudaMemcpyHostToDevice, c->stream));
-      c->h_scen_list = active;
-    }
+    TG_TRY(c->set_active(active));
     TG_TRY(c->run_graph(n, static_cast<int>(active.size())));
   }
   return TAPGPU_OK;
@@ -989,6 +1432,7 @@ int tapgpu_solve_begin(tapgpu_ctx* ctx, int max_iters, double target_relgap, con
   Ctx* c = ctx->c;
   TG_CUDA(cudaSetDevice(c->device));
   TG_TRY(c->ensure_scenarios(1));
+  TG_TRY(c->choose_paths(1));
   c->use_dem_scen = false;
   c->use_link_scen = false;
   TG_CUDA(cudaMemcpy(c->cap, c->h_cap.data(), sizeof(double) * c->M, cudaMemcpyHostToDevice));
@@ -1016,11 +1460,15 @@ int tapgpu_solve_advance(tapgpu_ctx* ctx, int max_new_iters, int* done, tapgpu_r
   TG_CUDA(cudaSetDevice(c->device));
   std::vector<tapgpu::ScenState> st;
   TG_TRY(c->read_states(1, st));
-  if (!st[0].done) {
-    int n = max_new_iters;
-    if (c->solve_max_iters > 0) n = std::max(1, std::min(n, c->solve_max_iters - st[0].iter));
-    TG_TRY(c->run_graph(n, 1));
+  int n = max_new_iters;
+  if (c->solve_max_iters > 0) n = std::max(1, std::min(n, c->solve_max_iters - st[0].iter));
+  const int goal = st[0].iter + n;
+  while (!st[0].done && st[0].iter < goal) {  // (again after a pause)
+    TG_TRY(c->set_active({0}));
+    TG_TRY(c->run_graph(goal - st[0].iter, 1));
     TG_TRY(c->read_states(1, st));
+    TG_TRY(c->sync_check());
+    TG_TRY(c->resume_paused(1, st));
   }
   TG_TRY(c->sync_check());
   int e = 0;
@@ -1150,6 +1598,7 @@ int tapgpu_solve_scenarios(tapgpu_ctx* ctx, int num_scen, const int64_t* scen_pt
   }
   TG_CUDA(cudaSetDevice(c->device));
   TG_TRY(c->ensure_scenarios(num_scen));
+  TG_TRY(c->choose_paths(num_scen));
   c->use_dem_scen = c->dem_scen == num_scen;
   c->use_link_scen = c->link_scen == num_scen;
   c->last_nscen = num_scen;
@@ -1242,22 +1691,24 @@ int tapgpu_solve_scenarios(tapgpu_ctx* ctx, int num_scen, const int64_t* scen_pt
     TG_TRY(c->enqueue_initial(num_scen, true));
   } else if (c->use_dem_scen || c->use_link_scen) {
     // every scenario has its own demand or links: load each at its own free flow
-    tapgpu::LinkArgs la = c->link_args(num_scen);
-    TG_CUDA(tapgpu::launch_set_costs(la, c->link_grid, c->stream));
-    TG_TRY(c->enqueue_paths(num_scen, true, c->e32, c->r32, c->w64, c->yfx, true));
-    la.pass = 0;
-    TG_CUDA(tapgpu::launch_init_flows(la, c->link_grid, c->stream));
+    TG_TRY(c->enqueue_initial(num_scen, false));
   } else {
     // free-flow all-or-nothing does not depend on capacity: load scenario 0
     // once and start every scenario from it
-    tapgpu::LinkArgs la = c->link_args(1);
-    TG_CUDA(tapgpu::launch_set_costs(la, c->link_grid, c->stream));
-    TG_TRY(c->enqueue_paths(1, true, c->e32, c->r32, c->w64, c->yfx, true));
+    TG_TRY(c->begin_paths(1));
+    if (c->hier_on && num_scen > 1) {  // its exponent too
+      std::vector<tapgpu::ScenState> st0;
+      TG_TRY(c->read_states(num_scen, st0));
+      for (int s = 1; s < num_scen; ++s) st0[s].u_exp = st0[0].u_exp;
+      TG_CUDA(cudaMemcpyAsync(c->state, st0.data(), sizeof(tapgpu::ScenState) * num_scen,
+                              cudaMemcpyHostToDevice, c->stream));
+      TG_CUDA(cudaStreamSynchronize(c->stream));
+    }
     for (int s = 1; s < num_scen; ++s)
       TG_CUDA(cudaMemcpyAsync(c->yfx + static_cast<size_t>(s) * M, c->yfx,
                               sizeof(unsigned long long) * M, cudaMemcpyDeviceToDevice,
                               c->stream));
-    la = c->link_args(num_scen);
+    tapgpu::LinkArgs la = c->link_args(num_scen);
     la.pass = 0;
     TG_CUDA(tapgpu::launch_init_flows(la, c->link_grid, c->stream));
   }
@@ -1278,6 +1729,8 @@ int tapgpu_set_scenario_demand(tapgpu_ctx* ctx, int num_scen, const double* dema
   TG_CUDA(cudaStreamSynchronize(c->stream));
   if (c->sc_od_q) tapgpu::free_owned(c, c->sc_od_q);
   if (c->sc_total) tapgpu::free_owned(c, c->sc_total);
+  if (c->h_sc_dem) tapgpu::free_owned(c, c->h_sc_dem);
+  c->h_sc_dem = nullptr;
   c->sc_od_q = nullptr;
   c->sc_total = nullptr;
   c->dem_scen = 0;
@@ -1324,6 +1777,7 @@ int tapgpu_set_scenario_demand(tapgpu_ctx* ctx, int num_scen, const double* dema
     TG_CUDA(cudaMemcpy(c->od_q, oq.data(), sizeof(long long) * nnz, cudaMemcpyHostToDevice));
     c->scale_bits = bits;
     c->inv_scale = std::ldexp(1.0, -bits);
+    if (c->hier) TG_TRY(c->hier_demand(c->od_q, 1, &c->h_dem));
   }
   const double scale = std::ldexp(1.0, c->scale_bits);
   std::vector<long long> q(static_cast<size_t>(num_scen) * nnz);
@@ -1332,6 +1786,7 @@ int tapgpu_set_scenario_demand(tapgpu_ctx* ctx, int num_scen, const double* dema
   TG_TRY(c->alloc_n(&c->sc_total, static_cast<size_t>(num_scen)));
   TG_CUDA(cudaMemcpy(c->sc_od_q, q.data(), sizeof(long long) * q.size(), cudaMemcpyHostToDevice));
   TG_CUDA(cudaMemcpy(c->sc_total, totals.data(), sizeof(double) * num_scen, cudaMemcpyHostToDevice));
+  if (c->hier) TG_TRY(c->hier_demand(c->sc_od_q, num_scen, &c->h_sc_dem));
   c->dem_scen = num_scen;
   return TAPGPU_OK;
 }
@@ -1661,18 +2116,31 @@ int tapgpu_run_iterations(tapgpu_ctx* ctx, int iters) {
                           cudaMemcpyHostToDevice, c->stream));
   std::vector<int> all(S);
   std::iota(all.begin(), all.end(), 0);
-  if (c->h_scen_list != all) {
-    TG_CUDA(cudaMemcpyAsync(c->scen_list, all.data(), sizeof(int) * S, cudaMemcpyHostToDevice,
-                            c->stream));
-    c->h_scen_list = all;
-  }
+  TG_TRY(c->set_active(all));
   int per = c->opt.iters_per_launch > 0 ? c->opt.iters_per_launch : 8;
   for (int done = 0; done < iters;) {
     const int n = std::min(per, iters - done);
     TG_TRY(c->run_graph(n, S));
     done += n;
   }
-  return TAPGPU_OK;
+  if (!c->hier_on) return TAPGPU_OK;
+  for (;;) {  // scenarios that paused on the way take their remaining iterations
+    TG_TRY(c->read_states(S, st));
+    bool paused = false;
+    for (auto& s : st) paused |= s.done > 1;
+    if (!paused) return TAPGPU_OK;
+    TG_TRY(c->resume_paused(S, st));
+    std::vector<int> active;
+    int left = 0;
+    for (int s = 0; s < S; ++s)
+      if (!st[s].done) {
+        active.push_back(s);
+        left = std::max(left, st[s].max_iters - st[s].iter);
+      }
+    if (active.empty()) return TAPGPU_OK;
+    TG_TRY(c->set_active(active));
+    TG_TRY(c->run_graph(std::max(1, std::min(per, left)), static_cast<int>(active.size())));
+  }
 }
 
 int tapgpu_set_timing(tapgpu_ctx* ctx, int on) {
@@ -1741,6 +2209,11 @@ int tapgpu_profile_iteration(tapgpu_ctx* ctx, int reps, float* ms) {
   for (int r = 0; r < reps && rc == TAPGPU_OK; ++r) {
     cudaEventRecord(ev[0], c->stream);
     const int64_t tasks = c->Z;
+    if (c->hier_on) {
+      rc = c->enqueue_hier(1, c->t, c->M, ev[1]);
+      if (rc != TAPGPU_OK) break;
+      cudaEventRecord(ev[2], c->stream);
+    } else {
     tapgpu::PathArgs a = c->path_args(1);
     a.task_end = static_cast<int>(tasks);
     cudaMemsetAsync(c->counters, 0, 2 * sizeof(int), c->stream);
@@ -1761,6 +2234,7 @@ int tapgpu_profile_iteration(tapgpu_ctx* ctx, int reps, float* ms) {
     tapgpu::launch_aon(a, c->fp64, std::min<int64_t>(c->aon_grid, tasks), c->aon_block,
                        c->aon_smem, c->stream);
     cudaEventRecord(ev[2], c->stream);
+    }
     tapgpu::LinkArgs la = c->link_args(1);
     for (int p = 0; p < tapgpu::kLsPasses; ++p) {
       la.pass = p;

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "fw_kernels.cuh"
+#include "hier_kernels.cuh"
 #include "tap_gpu.h"
 
 namespace tapgpu {
@@ -129,6 +130,30 @@ struct Ctx {
   double* api_w64 = nullptr;
   unsigned long long* api_yfx = nullptr;
 
+  // elimination hierarchy (hierarchy.h): the solver's shortest paths and
+  // loading where the plan suits the network; the label-correction kernels
+  // otherwise, and for a scenario whose labels leave the integers' range
+  bool hier = false;             // its plan is in place
+  bool hier_on = false;          // the iterations run on it (choose_paths)
+  int hier_cap = 0;              // scenarios that its buffers were made for
+  HierGraph hg{};
+  double hier_relaxations = 0;
+  std::vector<int> h_tile_ptr;   // first tile of each elimination level
+  int u_exp0 = 0;                // exponent of the first labels
+  int *h_opos = nullptr, *h_group = nullptr, *h_column = nullptr;  // origins by position
+  int *h_chain_ptr = nullptr, *h_chain = nullptr;
+  int* h_od_dest = nullptr;      // destination index of each OD entry or -1
+  int h_dests = 0, h_width = 0;  // demand by destination: [h_dests][h_width]
+  unsigned long long *h_dem = nullptr, *h_sc_dem = nullptr;
+  int hier_slots = 0;            // scenarios the buffers below hold
+  unsigned long long *h_w = nullptr, *h_d0 = nullptr, *h_fup = nullptr;
+  unsigned long long *h_dlab = nullptr, *h_vol = nullptr;
+  unsigned long long *h_mid = nullptr, *h_flow = nullptr;
+  unsigned char* h_via = nullptr;
+  int *h_from = nullptr, *h_list = nullptr, *h_list_n = nullptr;
+  unsigned short* h_arr = nullptr;
+  std::vector<std::pair<int, int>> hier_retry;  // per scenario: iteration, pauses in it
+
   cudaStream_t stream = nullptr;
   cudaGraphExec_t gexec = nullptr;
   int g_iters = 0, g_nscen = -1;
@@ -194,14 +219,27 @@ struct Ctx {
   }
   Demand demand() const;
   PathArgs path_args(int nscen_slots) const;
-  LinkArgs link_args(int nscen) const;
+  LinkArgs link_args(int nscen, bool records = false) const;
 
   // enqueue helpers (stream ordered, capturable)
   int enqueue_paths(int nscen, bool load, const uint2* e32p, const uint2* r32p, const double* w64p,
                     unsigned long long* ydst, bool use_state);
   int enqueue_iteration(int nscen);
   int enqueue_initial(int nscen, bool warm);
+  int enqueue_tail(int nscen);
   int run_graph(int iters, int nscen);
+  int hier_plan(const HierPlan* plan, const std::vector<int>& odest, const std::vector<int>& optr,
+                const std::vector<double>& odem);
+  int hier_demand(const long long* dev_q, int nscen, unsigned long long** dem);
+  void release_hier();
+  int ensure_hier(int S);
+  bool hier_pays(int nscen, int levels, double relaxations, int arcs) const;
+  int choose_paths(int nscen);
+  int ensure_legacy(int S);
+  int enqueue_hier(int nscen, const double* cost, long long stride, cudaEvent_t between = nullptr);
+  int begin_paths(int nscen);
+  int set_active(const std::vector<int>& active);
+  int resume_paused(int S, std::vector<ScenState>& st);
   int sync_check();
   int read_states(int S, std::vector<ScenState>& out);
 };
