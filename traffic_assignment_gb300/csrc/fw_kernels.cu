@@ -1791,6 +1791,39 @@ __device__ __forceinline__ void block_sum(double (&v)[N], double* sh /* [N][BLOC
   }
 }
 
+// Sixteen sums over a warp, sum (lane >> 1) in every lane: each step sends away
+// the half of the sums that the other half of the lanes keeps, 16 additions
+// instead of 80 (a warp's FP64 addition holds the unit for 16 cycles; a block
+// of 8 warps spent 5 us of a 107 us pass on them).
+__device__ __forceinline__ double warp_sum16(double (&v)[16]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16, n = 8; o >= 2; o >>= 1, n >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const double keep = up ? v[i + n] : v[i], send = up ? v[i] : v[i + n];
+      v[i] = __dadd_rn(keep, __shfl_xor_sync(kFull, send, o));
+    }
+  }
+  return __dadd_rn(v[0], __shfl_xor_sync(kFull, v[0], 1));
+}
+
+// Sixteen sums over a block: sum i in thread i.
+template <int BLOCK>
+__device__ __forceinline__ double block_sum16(double (&v)[16], double* sh /* [16][BLOCK/32] */) {
+  constexpr int W = BLOCK / 32;
+  const int lane = threadIdx.x & 31;
+  const double s = warp_sum16(v);
+  if (!(lane & 1)) sh[(lane >> 1) * W + (threadIdx.x >> 5)] = s;
+  __syncthreads();
+  double r = 0.0;
+  if (threadIdx.x < 16)
+#pragma unroll
+    for (int w = 0; w < W; ++w) r = __dadd_rn(r, sh[threadIdx.x * W + w]);
+  return r;
+}
+
 __device__ __forceinline__ int scen_of(const LinkArgs& a) {
   return a.scen_list ? a.scen_list[blockIdx.y] : static_cast<int>(blockIdx.y);
 }
@@ -1991,12 +2024,19 @@ __device__ __forceinline__ void ls_link(const LinkArgs& a, int scen, size_t off,
   const size_t pk = lpi(a.lp, scen, k);
   const double fft = a.lp.fft[pk], al = a.lp.alpha[pk], be = a.lp.beta[pk], c = cap[k];
   const unsigned char ip = a.lp.ipow[pk];
-  // FP32-path mode, integer power: t(x + lam d) = fft + (fft alpha) (x/c + lam d/c)^beta
-  // with one division per link (FP64 mode keeps the reference's forms,
-  // tap/tap_functions.c:55-65, 112-126)
-  const bool ratio = a.ls_ratio && ip != 255;
-  const double ic = ratio ? 1.0 / c : 0.0;
+  // integer power: t(x + lam d) = fft + (fft alpha) (x/c + lam d/c)^beta, with
+  // two divisions per link instead of one per candidate (a division is some
+  // 20 FP64 instructions, and an SM does two a clock; 40,000 links: 107 -> 34
+  // us per pass, with warp_sum16 and an even share of links).  The two
+  // quotients and the multiply-add round as often as the reference's product,
+  // sum and quotient (tap/tap_functions.c:55-65).  FP32-path mode takes one
+  // division, and the objective's term by the same form (FP64 mode: the
+  // reference's, tap/tap_functions.c:112-126).
+  const bool ratio = ip != 255;
+  const double ic = ratio && a.ls_ratio ? 1.0 / c : 0.0;
   const double A = fft * al;
+  const double r0 = !ratio ? 0.0 : (a.ls_ratio ? x * ic : __ddiv_rn(x, c));
+  double rd = 0.0;
   double d;
   if (pass == 0) {
     const double y = static_cast<double>(static_cast<long long>(a.y_fx[off + k])) * a.inv_scale;
@@ -2006,26 +2046,23 @@ __device__ __forceinline__ void ls_link(const LinkArgs& a, int scen, size_t off,
     const double t = a.t[off + k];
     acc[0] = __dadd_rn(acc[0], __dmul_rn(t, d));
     acc[1] = __dadd_rn(acc[1], __dmul_rn(x, t));
-    if (ratio) {
-      // x fft (1 + alpha / (beta + 1) (x/c)^beta) and t(x + d) d
-      const double r0 = x * ic;
-      acc[2] += x * (fft + A * bprf::int_pow_fast(r0, ip) * bprf::inv_int(ip + 1));
-      acc[3] += (fft + A * bprf::int_pow_fast(r0 + d * ic, ip)) * d;
-    } else {
-      acc[2] = __dadd_rn(acc[2], integral(fft, al, be, ip, c, x));
-      acc[3] = __dadd_rn(acc[3], __dmul_rn(bpr(fft, al, be, ip, c, __dadd_rn(x, d)), d));
-    }
+    acc[2] = a.ls_ratio && ratio
+                 ? acc[2] + x * (fft + A * bprf::int_pow_fast(r0, ip) * bprf::inv_int(ip + 1))
+                 : __dadd_rn(acc[2], integral(fft, al, be, ip, c, x));
   } else {
     d = a.d[off + k];
   }
   if (ratio) {
-    const double r0 = x * ic, rd = d * ic;
+    rd = a.ls_ratio ? d * ic : __ddiv_rn(d, c);
+    if (pass == 0) acc[3] += (fft + A * bprf::int_pow_fast(r0 + rd, ip)) * d;
 #pragma unroll
     for (int j = 0; j < kLsPerPass; ++j) {
       const double lam = ls_candidate(a.ls_mode, e0, blo, bhi, j);
       acc[4 + j] += (fft + A * bprf::int_pow_fast(r0 + lam * rd, ip)) * d;
     }
   } else {
+    if (pass == 0)
+      acc[3] = __dadd_rn(acc[3], __dmul_rn(bpr(fft, al, be, ip, c, __dadd_rn(x, d)), d));
 #pragma unroll
     for (int j = 0; j < kLsPerPass; ++j) {
       const double lam = ls_candidate(a.ls_mode, e0, blo, bhi, j);
@@ -2033,6 +2070,14 @@ __device__ __forceinline__ void ls_link(const LinkArgs& a, int scen, size_t off,
       acc[4 + j] = __dadd_rn(acc[4 + j], __dmul_rn(bpr(fft, al, be, ip, c, q), d));
     }
   }
+}
+
+// A block's links: an equal share in whole warps (the FP64 units of the SM with
+// the most links set the time).
+__device__ __forceinline__ void link_chunk(int m, int& k0, int& k1) {
+  const int per = ((m + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x) + 31) & ~31;
+  k0 = min(m, per * static_cast<int>(blockIdx.x));
+  k1 = min(m, k0 + per);
 }
 
 // One line-search pass; pass 0 also forms d = y - x and the gap / objective /
@@ -2053,14 +2098,13 @@ __global__ void __launch_bounds__(BLOCK) k_ls_pass(LinkArgs a) {
 #pragma unroll
   for (int i = 0; i < kNumSums; ++i) acc[i] = 0.0;
   const double* cap = a.cap + off;
-  for (int k = blockIdx.x * BLOCK + threadIdx.x; k < a.m; k += gridDim.x * BLOCK)
+  int k0, k1;
+  link_chunk(a.m, k0, k1);
+  for (int k = k0 + threadIdx.x; k < k1; k += BLOCK)
     ls_link(a, scen, off, cap, k, a.pass, e0, blo, bhi, acc);
-  block_sum<kNumSums, BLOCK>(acc, sh);
+  const double sum = block_sum16<BLOCK>(acc, sh);
   double* part = a.partials + (static_cast<size_t>(scen) * gridDim.x + blockIdx.x) * kNumSums;
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int i = 0; i < kNumSums; ++i) part[i] = acc[i];
-  }
+  if (threadIdx.x < kNumSums) part[threadIdx.x] = sum;
   if (!last_block(a.arrive + scen)) return;
   // the blocks' sums in a fixed order: BLOCK / kNumSums threads share a sum's
   // blocks (one thread alone waited for one load after the other: 100 us of
@@ -2219,7 +2263,9 @@ __global__ void __launch_bounds__(BLOCK) k_step(LinkArgs a) {
   const TapeAt tp = tape_at(a, scen, it);
   const double* cap = a.cap + off;
   double acc[1] = {0.0};
-  for (int k = blockIdx.x * BLOCK + threadIdx.x; k < a.m; k += gridDim.x * BLOCK)
+  int k0, k1;
+  link_chunk(a.m, k0, k1);
+  for (int k = k0 + threadIdx.x; k < k1; k += BLOCK)
     acc[0] = __dadd_rn(acc[0], step_link(a, scen, off, cap, k, lam, tp));
   block_sum<1, BLOCK>(acc, sh);
   double* part = a.partials + (static_cast<size_t>(scen) * gridDim.x + blockIdx.x) * kNumSums;
@@ -2246,6 +2292,7 @@ __global__ void __launch_bounds__(BLOCK) k_step(LinkArgs a) {
 constexpr int kTailBlock = 256;
 __global__ void __launch_bounds__(kTailBlock) k_fw_tail_small(LinkArgs a) {
   __shared__ double sh[kNumSums * (kTailBlock / 32)];
+  __shared__ double tot[kNumSums];
   __shared__ int sh_found;
   const int scen = scen_of(a);
   ScenState& st = a.state[scen];
@@ -2262,9 +2309,11 @@ __global__ void __launch_bounds__(kTailBlock) k_fw_tail_small(LinkArgs a) {
 #pragma unroll
     for (int i = 0; i < kNumSums; ++i) acc[i] = 0.0;
     for (int k = threadIdx.x; k < a.m; k += kTailBlock) ls_link(a, scen, off, cap, k, pass, e0, blo, bhi, acc);
-    block_sum<kNumSums, kTailBlock>(acc, sh);
+    const double sum = block_sum16<kTailBlock>(acc, sh);
+    if (threadIdx.x < kNumSums) tot[threadIdx.x] = sum;
+    __syncthreads();
     if (threadIdx.x == 0)
-      ls_decide(st, acc, e0, pass, a.total_demand_s ? a.total_demand_s[scen] : a.total_demand,
+      ls_decide(st, tot, e0, pass, a.total_demand_s ? a.total_demand_s[scen] : a.total_demand,
                 a.ls_mode);
     __syncthreads();
   }

@@ -887,7 +887,7 @@ int Ctx::enqueue_tail(int nscen) {
   TG_CUDA(launch_ls_fallback(la, stream));
   TG_TRY(mark(2, false));
   TG_TRY(mark(3, true));
-  TG_CUDA(launch_step(la, ls_link_grid, ls_block, stream));
+  TG_CUDA(launch_step(la, step_grid(nscen), ls_block, stream));
   TG_TRY(mark(3, false));
   count_launches(passes + 2);
   return TAPGPU_OK;
@@ -2242,7 +2242,7 @@ int tapgpu_profile_iteration(tapgpu_ctx* ctx, int reps, float* ms) {
     }
     tapgpu::launch_ls_fallback(la, c->stream);
     cudaEventRecord(ev[3], c->stream);
-    tapgpu::launch_step(la, c->ls_link_grid, c->ls_block, c->stream);
+    tapgpu::launch_step(la, c->step_grid(1), c->ls_block, c->stream);
     cudaEventRecord(ev[4], c->stream);
     if (cudaEventSynchronize(ev[4]) != cudaSuccess) {
       rc = TAPGPU_ERR_CUDA;

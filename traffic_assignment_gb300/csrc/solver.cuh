@@ -195,7 +195,14 @@ struct Ctx {
   // block reductions stay a small part of the FP64 work
   int ls_grid(int nscen) const {
     const int want = (16 * num_sms + nscen - 1) / (nscen > 0 ? nscen : 1);
-    return want < 1 ? 1 : (want > ls_link_grid ? ls_link_grid : want);
+    return want < 1 ? 1 : (want > step_grid(nscen) ? step_grid(nscen) : want);
+  }
+  // One scenario whose links make a few more blocks than there are SMs: one
+  // block per SM, its share a little longer (40,000 links: 157 blocks gave five
+  // SMs twice the FP64 work).
+  int step_grid(int nscen) const {
+    return nscen == 1 && ls_link_grid > num_sms && 4 * ls_link_grid < 5 * num_sms ? num_sms
+                                                                                  : ls_link_grid;
   }
 
   std::vector<DevMem> owned;
