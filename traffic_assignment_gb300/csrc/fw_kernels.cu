@@ -2695,6 +2695,25 @@ cudaError_t launch_fill_records4(uint4* p, size_t n, uint4 val, int grid, cudaSt
   return cudaGetLastError();
 }
 
+__global__ void __launch_bounds__(256) k_tree_rows(double* dist, size_t labels, const int* pred,
+                                                   const int64_t* perm, int64_t* out, size_t preds) {
+  const size_t i0 = static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x;
+  for (size_t i = i0; i < labels; i += static_cast<size_t>(gridDim.x) * 256)
+    if (isinf(dist[i])) dist[i] = DBL_MAX;
+  for (size_t i = i0; i < preds; i += static_cast<size_t>(gridDim.x) * 256) {
+    const int p = pred[i];
+    out[i] = p >= 0 ? __ldg(reinterpret_cast<const long long*>(perm) + p) : -1;
+  }
+}
+
+cudaError_t launch_tree_rows(double* dist, size_t labels, const int* pred, const int64_t* perm,
+                             int64_t* out, size_t preds, cudaStream_t s) {
+  const size_t n = std::max<size_t>(1, std::max(labels, preds));
+  const int grid = static_cast<int>(std::min<size_t>((n + 1023) / 1024, 1216));
+  k_tree_rows<<<grid, 256, 0, s>>>(dist, labels, pred, perm, out, preds);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_replicate_rows(double* x, int m, int nscen, int grid, cudaStream_t s) {
   if (nscen < 2) return cudaSuccess;
   k_replicate_rows<<<dim3(grid, nscen - 1), kLinkBlock, 0, s>>>(x, m);

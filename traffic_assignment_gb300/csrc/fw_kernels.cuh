@@ -219,6 +219,10 @@ cudaError_t launch_param_rows(unsigned char* rows, const unsigned char* base, in
                               const int* ptr, const int* link, const unsigned char* val, int grid,
                               cudaStream_t s);
 // rows 1 .. nscen-1 of x [nscen][m] become copies of row 0
+// the shortest-path API's results: labels in place (out of reach: DBL_MAX) and
+// predecessors as the caller's link indices (none: -1)
+cudaError_t launch_tree_rows(double* dist, size_t labels, const int* pred, const int64_t* perm,
+                             int64_t* out, size_t preds, cudaStream_t s);
 cudaError_t launch_replicate_rows(double* x, int m, int nscen, int grid, cudaStream_t s);
 cudaError_t launch_fill_records(uint2* p, size_t n, uint2 val, int grid, cudaStream_t s);
 cudaError_t launch_fill_records4(uint4* p, size_t n, uint4 val, int grid, cudaStream_t s);

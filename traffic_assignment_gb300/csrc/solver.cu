@@ -391,10 +391,6 @@ int Ctx::ensure_legacy(int S) {
       dist = nullptr;
       TG_TRY(alloc(&dist, static_cast<size_t>(tb) * static_cast<size_t>(want)));
       dist_tasks = want;
-      if (pred_buf) {  // sized by the label buffer: made again on its next use
-        free_owned(this, pred_buf);
-        pred_buf = nullptr;
-      }
     }
   }
   return TAPGPU_OK;
@@ -1296,6 +1292,7 @@ static int create_impl(const tapgpu_network* net, const tapgpu_demand* dem,
   TG_TRY(c->alloc(&c->dist, tb * c->dist_tasks));
   TG_TRY(c->alloc_n(&c->api_e32, M));
   TG_TRY(c->alloc_n(&c->api_e4, static_cast<size_t>(n1) * 4));
+  TG_CUDA(cudaMemset(c->api_e4, 0, sizeof(uint2) * static_cast<size_t>(n1) * 4));
   TG_TRY(c->alloc_n(&c->api_r32, M));
   TG_TRY(c->alloc_n(&c->api_w64, M));
   TG_TRY(c->alloc_n(&c->api_yfx, M));
@@ -1491,6 +1488,15 @@ int tapgpu_solve(tapgpu_ctx* ctx, int max_iters, double target_relgap, const dou
   return TAPGPU_OK;
 }
 
+// Writes to each page of an output array before the device copies to it: a page
+// that is not there yet costs the device's copy a fault (20 MB of fresh pages:
+// 1 to 17 ms; written by the host first, 0.8 ms and a copy of 0.15 ms).
+static void touch_pages(void* p, size_t bytes) {
+  auto* b = static_cast<volatile unsigned char*>(p);
+  for (size_t i = 0; i < bytes; i += 4096) b[i] = 0;
+  if (bytes) b[bytes - 1] = 0;
+}
+
 int tapgpu_get_link_flows(tapgpu_ctx* ctx, int scenario, double* volume, double* cost) {
   if (!ctx) return TAPGPU_ERR_ARG;
   Ctx* c = ctx->c;
@@ -1527,6 +1533,7 @@ int tapgpu_get_link_flows_batch(tapgpu_ctx* ctx, int first, int count, double* v
   for (int a = 0; a < 2; ++a) {
     if (!outs[a]) continue;
     if (identity) {  // the caller's link order is the device's: one copy
+      touch_pages(outs[a], sizeof(double) * n);
       TG_CUDA(cudaMemcpy(outs[a], srcs[a], sizeof(double) * n, cudaMemcpyDeviceToHost));
       continue;
     }
@@ -1920,9 +1927,11 @@ int tapgpu_set_scenario_links(tapgpu_ctx* ctx, int num_scen, const int64_t* edit
   return TAPGPU_OK;
 }
 
-static int to_device_weights(Ctx* c, const double* weights) {
-  std::vector<double> w(c->M);
-  std::vector<uint2> wf(c->M), wr(c->M);
+// The link costs of a call, in device order in api_w64, and the records of the
+// FP32 kernels made from them.  w stays until the stream has been waited for.
+static int to_device_weights(Ctx* c, const double* weights, std::vector<double>& w) {
+  w.resize(c->M);
+  double sum = 0.0;
   for (int k = 0; k < c->M; ++k) {
     const double v = weights[c->perm[k]];
     if (!(v >= 0) || std::isinf(v)) {
@@ -1930,30 +1939,25 @@ static int to_device_weights(Ctx* c, const double* weights) {
       return TAPGPU_ERR_ARG;
     }
     w[k] = v;
-    const float f = static_cast<float>(v);
-    unsigned bits;
-    std::memcpy(&bits, &f, sizeof bits);
-    wf[k] = make_uint2(static_cast<unsigned>(c->h_head[k]), bits);
-    wr[c->h_rpos[k]] = make_uint2(static_cast<unsigned>(c->h_tail[k]), bits);
+    sum += v;
   }
-  {
-    double s = 0.0;
-    for (int k = 0; k < c->M; ++k) s += w[k];
-    const double mean = s / c->M;
-    c->api_nf_delta = c->opt.nf_delta > 0 ? c->opt.nf_delta : (mean > 0 ? 16.0 * mean : 1.0);
-  }
-  TG_CUDA(cudaMemcpyAsync(c->api_r32, wr.data(), sizeof(uint2) * c->M, cudaMemcpyHostToDevice,
-                          c->stream));
+  const double mean = sum / c->M;
+  c->api_nf_delta = c->opt.nf_delta > 0 ? c->opt.nf_delta : (mean > 0 ? 16.0 * mean : 1.0);
   TG_CUDA(cudaMemcpyAsync(c->api_w64, w.data(), sizeof(double) * c->M, cudaMemcpyHostToDevice,
                           c->stream));
-  TG_CUDA(cudaMemcpyAsync(c->api_e32, wf.data(), sizeof(uint2) * c->M, cudaMemcpyHostToDevice,
-                          c->stream));
-  std::vector<uint2> w4(static_cast<size_t>(c->n1) * 4, make_uint2(0u, 0u));
-  for (int k = 0; k < c->M; ++k)
-    if (c->h_ell_pos[k] >= 0) w4[c->h_ell_pos[k]] = make_uint2(c->h_e4x[k], wf[k].y);
-  TG_CUDA(cudaMemcpyAsync(c->api_e4, w4.data(), sizeof(uint2) * w4.size(), cudaMemcpyHostToDevice,
-                          c->stream));
-  TG_CUDA(cudaStreamSynchronize(c->stream));
+  if (!c->fp64) {
+    tapgpu::LinkArgs la = c->link_args(1);
+    la.scen_list = nullptr;
+    la.absent = nullptr;
+    la.t = c->api_w64;
+    la.w64 = nullptr;
+    la.e32 = c->api_e32;
+    la.r32 = c->api_r32;
+    la.e4 = c->api_e4;
+    la.r4 = nullptr;
+    la.r4d = nullptr;
+    TG_CUDA(tapgpu::launch_records(la, c->link_grid, c->stream));
+  }
   return TAPGPU_OK;
 }
 
@@ -1967,30 +1971,43 @@ int tapgpu_sssp(tapgpu_ctx* ctx, const double* weights, const int64_t* srcs, int
       return TAPGPU_ERR_ARG;
     }
   TG_CUDA(cudaSetDevice(c->device));
-  TG_TRY(to_device_weights(c, weights));
+  std::vector<double> w;
+  TG_TRY(to_device_weights(c, weights, w));
   const int n1 = c->n1;
-  if (!c->pred_buf) TG_TRY(c->alloc_n(&c->pred_buf, static_cast<size_t>(c->dist_tasks) * n1));
-  int* dsrc = nullptr;
   // FP64 labels: a FP32 context's label buffer holds half as many sources
   const int64_t chunk = c->fp64 ? c->dist_tasks : std::max<int64_t>(1, c->dist_tasks / 2);
-  TG_TRY(c->alloc_n(&dsrc, static_cast<size_t>(std::max<int64_t>(1, std::min(chunk, num_sources)))));
-  std::vector<double> dtmp;
-  std::vector<float> ftmp;
-  std::vector<int> ptmp;
+  const int64_t rows = std::max<int64_t>(1, std::min(chunk, num_sources));
+  if (rows > c->api_rows) {  // sources, predecessors and their wide form
+    void* olds[] = {c->api_src, c->pred_buf, c->api_pred};
+    for (void* p : olds) tapgpu::free_owned(c, p);
+    c->api_src = c->pred_buf = nullptr;
+    c->api_pred = nullptr;
+    c->api_rows = 0;
+    c->api_pred_rows = std::max<int64_t>(1, std::min<int64_t>(rows, (int64_t(64) << 20) / (8 * n1)));
+    TG_TRY(c->alloc_n(&c->api_src, static_cast<size_t>(rows)));
+    TG_TRY(c->alloc_n(&c->pred_buf, static_cast<size_t>(rows) * n1));
+    TG_TRY(c->alloc_n(&c->api_pred, static_cast<size_t>(c->api_pred_rows) * n1));
+    if (!c->api_perm) {
+      TG_TRY(c->alloc_n(&c->api_perm, static_cast<size_t>(c->M)));
+      TG_CUDA(cudaMemcpy(c->api_perm, c->perm.data(), sizeof(int64_t) * c->M, cudaMemcpyHostToDevice));
+    }
+    c->api_rows = rows;
+  }
+  std::vector<int> hs;
   int rc = TAPGPU_OK;
   // the API always computes FP64 labels: they equal the reference's bit for bit
   for (int64_t s0 = 0; s0 < num_sources && rc == TAPGPU_OK; s0 += chunk) {
     const int64_t s1 = std::min(num_sources, s0 + chunk);
     const int ns = static_cast<int>(s1 - s0);
-    std::vector<int> hs(ns);
+    hs.resize(ns);
     for (int i = 0; i < ns; ++i) hs[i] = static_cast<int>(srcs[s0 + i]);
-    if (cudaMemcpyAsync(dsrc, hs.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, c->stream) !=
+    if (cudaMemcpyAsync(c->api_src, hs.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, c->stream) !=
         cudaSuccess) {
       rc = TAPGPU_ERR_CUDA;
       break;
     }
     tapgpu::PathArgs a = c->path_args(1);
-    a.sources = dsrc;
+    a.sources = c->api_src;
     a.num_sources = ns;
     a.scen_list = nullptr;
     a.state = nullptr;
@@ -2046,30 +2063,30 @@ int tapgpu_sssp(tapgpu_ctx* ctx, const double* weights, const int64_t* srcs, int
       rc = TAPGPU_ERR_CUDA;
       break;
     }
+    const size_t at = static_cast<size_t>(s0) * n1, count = static_cast<size_t>(ns) * n1;
+    const size_t step = pred ? static_cast<size_t>(c->api_pred_rows) * n1 : count;
+    if (tapgpu::launch_tree_rows(static_cast<double*>(c->dist), count, c->pred_buf, c->api_perm,
+                                 c->api_pred, pred ? std::min(step, count) : 0, c->stream) != cudaSuccess) {
+      rc = TAPGPU_ERR_CUDA;
+      break;
+    }
+    // (while the kernels run)
+    if (dist) touch_pages(dist + at, sizeof(double) * count);
+    if (pred) touch_pages(pred + at, sizeof(int64_t) * count);
     rc = c->sync_check();
     if (rc != TAPGPU_OK) break;
-    if (dist) {
-      dtmp.resize(static_cast<size_t>(ns) * n1);
-      if (cudaMemcpy(dtmp.data(), c->dist, sizeof(double) * dtmp.size(), cudaMemcpyDeviceToHost) !=
-          cudaSuccess) {
-        rc = TAPGPU_ERR_CUDA;
-        break;
-      }
-      for (size_t i = 0; i < dtmp.size(); ++i)
-        dist[static_cast<size_t>(s0) * n1 + i] = std::isinf(dtmp[i]) ? DBL_MAX : dtmp[i];
+    bool copied = !dist || cudaMemcpy(dist + at, c->dist, sizeof(double) * count,
+                                      cudaMemcpyDeviceToHost) == cudaSuccess;
+    for (size_t i = 0; pred && i < count && copied; i += step) {
+      const size_t n = std::min(step, count - i);
+      copied = (i == 0 || tapgpu::launch_tree_rows(nullptr, 0, c->pred_buf + i, c->api_perm, c->api_pred,
+                                                   n, c->stream) == cudaSuccess) &&
+               cudaStreamSynchronize(c->stream) == cudaSuccess &&
+               cudaMemcpy(pred + at + i, c->api_pred, sizeof(int64_t) * n, cudaMemcpyDeviceToHost) ==
+                   cudaSuccess;
     }
-    if (pred) {
-      ptmp.resize(static_cast<size_t>(ns) * n1);
-      if (cudaMemcpy(ptmp.data(), c->pred_buf, sizeof(int) * ptmp.size(), cudaMemcpyDeviceToHost) !=
-          cudaSuccess) {
-        rc = TAPGPU_ERR_CUDA;
-        break;
-      }
-      for (size_t i = 0; i < ptmp.size(); ++i)
-        pred[static_cast<size_t>(s0) * n1 + i] = ptmp[i] >= 0 ? c->perm[ptmp[i]] : -1;
-    }
+    if (!copied) rc = TAPGPU_ERR_CUDA;
   }
-  tapgpu::free_owned(c, dsrc);
   if (rc == TAPGPU_ERR_CUDA && tapgpu::g_message.empty())
     tapgpu::set_message(cudaGetErrorString(cudaGetLastError()));
   return rc;
@@ -2079,7 +2096,8 @@ int tapgpu_aon(tapgpu_ctx* ctx, const double* weights, double* volume) {
   if (!ctx || !weights || !volume) return TAPGPU_ERR_ARG;
   Ctx* c = ctx->c;
   TG_CUDA(cudaSetDevice(c->device));
-  TG_TRY(to_device_weights(c, weights));
+  std::vector<double> w;
+  TG_TRY(to_device_weights(c, weights, w));
   TG_CUDA(cudaMemsetAsync(c->api_yfx, 0, sizeof(unsigned long long) * c->M, c->stream));
   TG_CUDA(cudaMemsetAsync(c->err, 0, sizeof(int), c->stream));
   const double solver_delta = c->nf_delta;

@@ -121,7 +121,11 @@ struct Ctx {
   int* counters = nullptr;  // [2]
   int* err = nullptr;       // [1]
   int* err_info = nullptr;  // [2]
-  int* pred_buf = nullptr;  // [dist_tasks][n1] for the shortest-path API
+  // shortest-path API: sources, predecessors [api_rows][n1] and, api_pred_rows
+  // at a time, as the caller's link indices
+  int *api_src = nullptr, *pred_buf = nullptr;
+  int64_t *api_pred = nullptr, *api_perm = nullptr;
+  int64_t api_rows = 0, api_pred_rows = 0;
   unsigned long long* path_stats = nullptr;  // [8] rounds, tasks, expansions, idle polls, batches
   // buffers of the one-shot API (weights in both precisions, loaded volumes)
   uint2* api_e32 = nullptr;
