@@ -1305,6 +1305,106 @@ __global__ void __launch_bounds__(BLOCK) k_sssp_small(PathArgs a) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// k_sssp_edges: the same sweeps with the edges in registers
+// ---------------------------------------------------------------------------
+// A thread holds NPE edges and the tail label that each was last relaxed with:
+// a sweep is one shared-memory load per edge, and only an edge whose tail's
+// label is new goes on to the addition (FP64: 16 cycles of the unit per warp),
+// the head's label and the atomic.  The block meets once in kEdgeSweeps sweeps.
+// A sweep of k_sssp_small was a chain of six shared-memory accesses for every
+// edge and a barrier.  Per launch, FP32 / FP64: 416 nodes, 38 origins, one
+// scenario 35 -> 20 / 48 -> 30 us, 400 scenarios 820 -> 407 / 1350 -> 776 us;
+// 1,710 nodes, 60 origins 181 -> 70 / 232 -> 111 us.  (By node instead, pulling
+// over its in-links: 16 us for the first in FP32, but 60 to 90 in FP64, whose
+// additions it does not skip, and slower in batches.)  3 or 12 sweeps per
+// meeting are within 5 % of 6.
+constexpr int kEdgeSweeps = 6;
+constexpr int kEdgeMax = 8;  // per thread
+constexpr int kEdgeBlock = 512;
+
+template <typename T, int NPE>
+__global__ void __launch_bounds__(kEdgeBlock) k_sssp_edges(PathArgs a) {
+  constexpr int BLOCK = kEdgeBlock;
+  using U = typename DT<T>::U;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int sh_task;
+  U* dist = reinterpret_cast<U*>(smem_raw);  // [n1 + 1], the last one out of reach
+  const int n1 = a.g.n1, m = a.g.m, F = a.g.first_thru;
+  int tail[NPE], head[NPE];
+  T w[NPE];
+#pragma unroll
+  for (int i = 0; i < NPE; ++i) {
+    const int k = threadIdx.x + i * BLOCK;
+    tail[i] = k < m ? __ldg(a.g.tail + k) : n1;
+    head[i] = 0;
+    w[i] = T(0);
+  }
+  int staged = -1;  // scenario whose weights are in registers
+
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) sh_task = atomicAdd(a.counter, 1) + a.task_begin;
+    __syncthreads();
+    const int task = sh_task;
+    if (task >= a.task_end) break;
+    const int slot = task / a.num_sources;
+    const int scen = a.scen_list ? a.scen_list[slot] : 0;
+    if (a.state && a.state[scen].done) continue;
+    const int src = a.sources[task - slot * a.num_sources];
+    if (scen != staged) {  // (uniform)
+      const Edges<T> ed = edges_of<T>(a, scen);
+#pragma unroll
+      for (int i = 0; i < NPE; ++i) {
+        const int k = threadIdx.x + i * BLOCK;
+        if (k < m) ed.load(k, head[i], w[i]);
+      }
+      staged = scen;
+    }
+    for (int v = threadIdx.x; v <= n1; v += BLOCK) dist[v] = DT<T>::kInf;
+    __syncthreads();
+    if (threadIdx.x == 0) dist[src] = DT<T>::bits(T(0));
+    __syncthreads();
+    U seen[NPE];
+    int at[NPE];  // zones are never passed through
+#pragma unroll
+    for (int i = 0; i < NPE; ++i) {
+      seen[i] = DT<T>::kInf;
+      at[i] = tail[i] < F && tail[i] != src ? n1 : tail[i];
+    }
+    int sweeps = 0;
+    for (;;) {
+      int changed = 0;
+#pragma unroll 1
+      for (int p = 0; p < kEdgeSweeps; ++p) {
+        U du[NPE];
+#pragma unroll
+        for (int i = 0; i < NPE; ++i) du[i] = vload(dist + at[i]);
+#pragma unroll
+        for (int i = 0; i < NPE; ++i)
+          if (du[i] != seen[i]) {
+            seen[i] = du[i];
+            const U nb = DT<T>::bits(DT<T>::add(DT<T>::val(du[i]), w[i]));
+            if (nb < vload(dist + head[i]) && nb < atomicMin(dist + head[i], nb)) changed = 1;
+          }
+      }
+      sweeps += kEdgeSweeps;
+      if (!__syncthreads_or(changed)) break;
+      // (one link of a path at least each time the block meets)
+      if (sweeps > kEdgeSweeps * (n1 + 1)) {  // (cannot happen with non-negative weights)
+        if (threadIdx.x == 0) atomicOr(a.err, kErrRounds);
+        break;
+      }
+    }
+    T* out = static_cast<T*>(a.dist) + static_cast<size_t>(task - a.task_begin) * n1;
+    for (int v = threadIdx.x; v < n1; v += BLOCK) out[v] = DT<T>::val(dist[v]);
+    if (a.stats && threadIdx.x == 0) {
+      atomicAdd(a.stats + 0, static_cast<unsigned long long>(sweeps));
+      atomicAdd(a.stats + 1, 1ull);
+    }
+  }
+}
+
 constexpr unsigned short kNoParent16 = 0xffffu;  // node ids are below 65535 in the compact layout
 
 template <bool COMPACT>
@@ -2357,8 +2457,21 @@ cudaError_t allow_max_smem(Fn fn) {
 
 using PathKernel = void (*)(PathArgs);
 
+// the small networks' kernel by edges per thread (a caller's own block size
+// takes k_sssp_small)
+bool sssp_edges(int m, int variant, int block, bool smem) {
+  return variant == kSsspSmall && smem && block == kEdgeBlock && m <= kEdgeMax * kEdgeBlock;
+}
+
 template <typename T, int BLOCK, bool SMEM>
-PathKernel sssp_kernel(int variant) {
+PathKernel sssp_kernel(int variant, int m) {
+  if constexpr (BLOCK == kEdgeBlock && SMEM)
+    if (sssp_edges(m, variant, BLOCK, SMEM)) {
+      constexpr PathKernel fns[kEdgeMax] = {k_sssp_edges<T, 1>, k_sssp_edges<T, 2>, k_sssp_edges<T, 3>,
+                                            k_sssp_edges<T, 4>, k_sssp_edges<T, 5>, k_sssp_edges<T, 6>,
+                                            k_sssp_edges<T, 7>, k_sssp_edges<T, 8>};
+      return fns[(m - 1) / kEdgeBlock];
+    }
   if (variant == kSsspSmall) return k_sssp_small<T, BLOCK, SMEM>;
   if (variant == kSsspRounds) return k_sssp<T, BLOCK, SMEM>;
   if (variant == kSsspAsync) return k_sssp_async<T, BLOCK, SMEM>;
@@ -2382,7 +2495,8 @@ cudaError_t launch_sssp_t(const PathArgs& a, int grid, size_t smem, int variant,
     fn<<<grid, BLOCK, nfq_split_smem_bytes(a.g.n1, variant), s>>>(a);
     return cudaGetLastError();
   }
-  PathKernel fn = sssp_kernel<T, BLOCK, SMEM>(variant);
+  PathKernel fn = sssp_kernel<T, BLOCK, SMEM>(variant, a.g.m);
+  if (sssp_edges(a.g.m, variant, BLOCK, SMEM)) smem = align16(sizeof(T) * (a.g.n1 + 1));
   if (SMEM) {
     cudaError_t e = allow_max_smem(fn);
     if (e != cudaSuccess) return e;
@@ -2489,8 +2603,9 @@ cudaError_t launch_aon(const PathArgs& a, bool fp64, int grid, int block, bool s
 }
 
 template <typename T, int BLOCK, bool SMEM>
-int occ_sssp_t(size_t smem, int variant, int n1, bool all_global) {
-  PathKernel fn = sssp_kernel<T, BLOCK, SMEM>(variant);
+int occ_sssp_t(size_t smem, int variant, int n1, int m, bool all_global) {
+  PathKernel fn = sssp_kernel<T, BLOCK, SMEM>(variant, m);
+  if (sssp_edges(m, variant, BLOCK, SMEM)) smem = align16(sizeof(T) * (n1 + 1));
   if (!SMEM && !all_global && nfq_split(n1, variant)) {
     fn = nfq_split_kernel<T, BLOCK>(variant);
     smem = nfq_split_smem_bytes(n1, variant);
@@ -2520,10 +2635,10 @@ int sssp_occupancy(bool fp64, int block, bool smem, int n1, int variant, int m, 
   const size_t bytes = sssp_smem_bytes(n1, fp64, variant, m);
 #define TAPGPU_OCC(B)                                                                       \
   if (block == B) {                                                                         \
-    if (fp64) return smem ? occ_sssp_t<double, B, true>(bytes, variant, n1, all_global)     \
-                          : occ_sssp_t<double, B, false>(bytes, variant, n1, all_global);   \
-    return smem ? occ_sssp_t<float, B, true>(bytes, variant, n1, all_global)                \
-                : occ_sssp_t<float, B, false>(bytes, variant, n1, all_global);              \
+    if (fp64) return smem ? occ_sssp_t<double, B, true>(bytes, variant, n1, m, all_global)     \
+                          : occ_sssp_t<double, B, false>(bytes, variant, n1, m, all_global);   \
+    return smem ? occ_sssp_t<float, B, true>(bytes, variant, n1, m, all_global)                \
+                : occ_sssp_t<float, B, false>(bytes, variant, n1, m, all_global);              \
   }
   TAPGPU_OCC(128)
   TAPGPU_OCC(256)
