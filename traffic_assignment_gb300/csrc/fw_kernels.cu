@@ -2049,15 +2049,56 @@ __global__ void __launch_bounds__(kLinkBlock) k_records(LinkArgs a) {
     write_weights(a, scen, k, a.t[off + k]);
 }
 
-// candidate step j of a pass: 2^-(e0+j) (reference rule) or the j-th of 12
-// interior points of the current bracket (exact root)
-__device__ __forceinline__ double ls_candidate(int mode, int e0, double lo, double hi, int j) {
-  if (mode == kLsExact) return lo + (hi - lo) * static_cast<double>(j + 1) / (kLsPerPass + 1);
-  return pow2neg(e0 + j);
+// distances of the exact search's candidates from the root's estimate, as parts
+// of the way to the bracket's ends
+__device__ __forceinline__ double ls_part(int i) {
+  constexpr double part[6] = {0x1p-2, 0x1p-5, 0x1p-10, 0x1p-16, 0x1p-24, 0x1p-34};
+  return part[i];
 }
 
-__device__ void ls_decide(ScenState& st, const double* tot, int first_e, int pass, double total_demand,
-                          int mode) {
+// What a pass tries.  Reference rule: 2^-(e0+j).  Exact root, first pass: 12
+// even points of the bracket; then six on either side of the estimate, so that
+// the next bracket is about as small as the estimate's error.  A bracket that
+// did not become 13 times smaller is cut by even points again.  (Even points
+// only: 14 passes; now 5 or 6.)
+struct LsTry {
+  int mode, pass, e0;
+  double lo, hi, root;
+  __device__ __forceinline__ LsTry(const ScenState& st, int mode, int pass)
+      : mode(mode), pass(pass), e0(pass == 0 ? 1 : st.ls_next), lo(pass == 0 ? 0.0 : st.ls_lo),
+        hi(pass == 0 ? 1.0 : st.ls_hi), root(pass == 0 ? -1.0 : st.ls_root) {}
+  __device__ __forceinline__ double at(int j) const {
+    if (mode != kLsExact) return pow2neg(e0 + j);
+    if (root < 0) return lo + (hi - lo) * static_cast<double>(j + 1) / (kLsPerPass + 1);
+    static_assert(kLsPerPass == 12, "six on either side");
+    return j < 6 ? root - (root - lo) * ls_part(j) : root + (hi - root) * ls_part(11 - j);
+  }
+};
+
+// Estimate of the root of g from n points of rising g, the sign change between
+// i - 1 and i: inverse interpolation through up to four of them, the secant
+// where that leaves the bracket.
+__device__ inline double ls_estimate(const double* lam, const double* g, int n, int i) {
+  const double lo = lam[i - 1], hi = lam[i], den = g[i] - g[i - 1];
+  const int b = max(0, i - 2), m = min(n, i + 2) - b;
+  double p[4], r = lo;
+  bool rising = true;
+  for (int k = 0; k < m; ++k) {
+    p[k] = lam[b + k];
+    if (k > 0 && !(g[b + k] > g[b + k - 1])) rising = false;
+  }
+  if (rising) {  // Neville's scheme at g = 0
+    for (int w = 1; w < m; ++w)
+      for (int k = 0; k + w < m; ++k)
+        p[k] = (g[b + k + w] * p[k] - g[b + k] * p[k + 1]) / (g[b + k + w] - g[b + k]);
+    r = p[0];
+  }
+  if (!(r > lo && r < hi) && den > 0) r = lo + (hi - lo) * (-g[i - 1] / den);
+  return r > lo && r < hi ? r : 0.5 * (lo + hi);
+}
+
+__device__ void ls_decide(ScenState& st, const double* tot, const LsTry& tr, double total_demand) {
+  const int mode = tr.mode, pass = tr.pass, first_e = tr.e0;
   if (pass == 0) {
     const double g0 = tot[0];
     st.g0 = g0;
@@ -2086,17 +2127,24 @@ __device__ void ls_decide(ScenState& st, const double* tot, int first_e, int pas
   }
   if (mode == kLsExact) {
     // g rises with lambda (convex objective): keep the sign change bracketed
-    const double lo = st.ls_lo, hi = st.ls_hi;
+    double lam[kLsPerPass + 2], g[kLsPerPass + 2];
+    lam[0] = st.ls_lo;
+    g[0] = st.ls_glo;
     for (int j = 0; j < kLsPerPass; ++j) {
-      const double lam = ls_candidate(mode, 0, lo, hi, j);
-      if (tot[4 + j] > 0) {
-        st.ls_hi = lam;
-        st.ls_ghi = tot[4 + j];
-        break;
-      }
-      st.ls_lo = lam;
-      st.ls_glo = tot[4 + j];
+      lam[j + 1] = tr.at(j);
+      g[j + 1] = tot[4 + j];
     }
+    lam[kLsPerPass + 1] = st.ls_hi;
+    g[kLsPerPass + 1] = st.ls_ghi;
+    int i = 1;
+    while (i <= kLsPerPass && !(g[i] > 0)) ++i;
+    st.ls_lo = lam[i - 1];
+    st.ls_glo = g[i - 1];
+    st.ls_hi = lam[i];
+    st.ls_ghi = g[i];
+    st.ls_root = 13.0 * (st.ls_hi - st.ls_lo) <= (tr.hi - tr.lo) * (1.0 + 1e-9)
+                     ? ls_estimate(lam, g, kLsPerPass + 2, i)
+                     : -1.0;
     if (pass + 1 >= kLsExactPasses || st.ls_hi - st.ls_lo <= 1e-15 * st.ls_hi) {
       const double den = st.ls_glo - st.ls_ghi;
       st.lambda = den < 0 ? st.ls_lo + (st.ls_hi - st.ls_lo) * (st.ls_glo / den) : st.ls_lo;
@@ -2118,8 +2166,8 @@ __device__ void ls_decide(ScenState& st, const double* tot, int first_e, int pas
 // adds the link's gap, VHT, objective and g(1) terms; every pass adds its
 // candidate steps' terms.
 __device__ __forceinline__ void ls_link(const LinkArgs& a, int scen, size_t off, const double* cap,
-                                        int k, int pass, int e0, double blo, double bhi,
-                                        double (&acc)[kNumSums]) {
+                                        int k, const LsTry& tr, double (&acc)[kNumSums]) {
+  const int pass = tr.pass;
   const double x = a.x[off + k];
   const size_t pk = lpi(a.lp, scen, k);
   const double fft = a.lp.fft[pk], al = a.lp.alpha[pk], be = a.lp.beta[pk], c = cap[k];
@@ -2157,7 +2205,7 @@ __device__ __forceinline__ void ls_link(const LinkArgs& a, int scen, size_t off,
     if (pass == 0) acc[3] += (fft + A * bprf::int_pow_fast(r0 + rd, ip)) * d;
 #pragma unroll
     for (int j = 0; j < kLsPerPass; ++j) {
-      const double lam = ls_candidate(a.ls_mode, e0, blo, bhi, j);
+      const double lam = tr.at(j);
       acc[4 + j] += (fft + A * bprf::int_pow_fast(r0 + lam * rd, ip)) * d;
     }
   } else {
@@ -2165,7 +2213,7 @@ __device__ __forceinline__ void ls_link(const LinkArgs& a, int scen, size_t off,
       acc[3] = __dadd_rn(acc[3], __dmul_rn(bpr(fft, al, be, ip, c, __dadd_rn(x, d)), d));
 #pragma unroll
     for (int j = 0; j < kLsPerPass; ++j) {
-      const double lam = ls_candidate(a.ls_mode, e0, blo, bhi, j);
+      const double lam = tr.at(j);
       const double q = __dadd_rn(x, __dmul_rn(lam, d));
       acc[4 + j] = __dadd_rn(acc[4 + j], __dmul_rn(bpr(fft, al, be, ip, c, q), d));
     }
@@ -2191,9 +2239,7 @@ __global__ void __launch_bounds__(BLOCK) k_ls_pass(LinkArgs a) {
   if (st.done) return;
   if (a.pass > 0 && !st.ls_pending) return;
   const size_t off = static_cast<size_t>(scen) * a.m;
-  const int e0 = a.pass == 0 ? 1 : st.ls_next;
-  const double blo = a.pass == 0 ? 0.0 : st.ls_lo;
-  const double bhi = a.pass == 0 ? 1.0 : st.ls_hi;
+  const LsTry tr(st, a.ls_mode, a.pass);
   double acc[kNumSums];
 #pragma unroll
   for (int i = 0; i < kNumSums; ++i) acc[i] = 0.0;
@@ -2201,7 +2247,7 @@ __global__ void __launch_bounds__(BLOCK) k_ls_pass(LinkArgs a) {
   int k0, k1;
   link_chunk(a.m, k0, k1);
   for (int k = k0 + threadIdx.x; k < k1; k += BLOCK)
-    ls_link(a, scen, off, cap, k, a.pass, e0, blo, bhi, acc);
+    ls_link(a, scen, off, cap, k, tr, acc);
   const double sum = block_sum16<BLOCK>(acc, sh);
   double* part = a.partials + (static_cast<size_t>(scen) * gridDim.x + blockIdx.x) * kNumSums;
   if (threadIdx.x < kNumSums) part[threadIdx.x] = sum;
@@ -2229,8 +2275,7 @@ __global__ void __launch_bounds__(BLOCK) k_ls_pass(LinkArgs a) {
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    ls_decide(st, parts[0], e0, a.pass, a.total_demand_s ? a.total_demand_s[scen] : a.total_demand,
-              a.ls_mode);
+    ls_decide(st, parts[0], tr, a.total_demand_s ? a.total_demand_s[scen] : a.total_demand);
     a.arrive[scen] = 0u;
   }
 }
@@ -2284,11 +2329,36 @@ __device__ void ls_fallback_block(const LinkArgs& a, int scen, ScenState& st, do
   }
 }
 
-__global__ void __launch_bounds__(1024) k_ls_fallback(LinkArgs a) {
-  __shared__ double sh[32];
+// The passes from a.pass on by one block per scenario, for a search that the
+// passes over the whole grid left open (steps below 2^-24, of small networks
+// below 2^-12), and the halvings beyond them.  Launches that find nothing to do
+// cost 2 us each: one for all of them instead of one per pass.
+constexpr int kRestBlock = 512;
+__global__ void __launch_bounds__(kRestBlock) k_ls_rest(LinkArgs a) {
+  __shared__ double sh[kNumSums * (kRestBlock / 32)];
+  __shared__ double tot[kNumSums];
   __shared__ int sh_found;
   const int scen = scen_of(a);
-  ls_fallback_block(a, scen, a.state[scen], sh, &sh_found);
+  ScenState& st = a.state[scen];
+  if (st.done || !st.ls_pending) return;  // (read by every thread before any change to it)
+  const size_t off = static_cast<size_t>(scen) * a.m;
+  const double* cap = a.cap + off;
+  __syncthreads();
+  const int passes = a.ls_mode == kLsExact ? kLsExactPasses : kLsPasses;
+  for (int pass = a.pass; pass < passes && st.ls_pending; ++pass) {
+    const LsTry tr(st, a.ls_mode, pass);
+    double acc[kNumSums];
+#pragma unroll
+    for (int i = 0; i < kNumSums; ++i) acc[i] = 0.0;
+    for (int k = threadIdx.x; k < a.m; k += kRestBlock) ls_link(a, scen, off, cap, k, tr, acc);
+    const double sum = block_sum16<kRestBlock>(acc, sh);
+    if (threadIdx.x < kNumSums) tot[threadIdx.x] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0)
+      ls_decide(st, tot, tr, a.total_demand_s ? a.total_demand_s[scen] : a.total_demand);
+    __syncthreads();
+  }
+  ls_fallback_block(a, scen, st, sh, &sh_found);
 }
 
 // Where iteration `it` of a scenario writes its adjoint tape: every
@@ -2387,7 +2457,7 @@ __global__ void __launch_bounds__(BLOCK) k_step(LinkArgs a) {
 
 // Small networks: the whole tail of an iteration (every line-search pass,
 // the fallback, the step) by one 256-thread block per scenario, one launch
-// instead of seven; the same per-link arithmetic as k_ls_pass, k_ls_fallback
+// instead of seven; the same per-link arithmetic as k_ls_pass, k_ls_rest
 // and k_step, with block-wide sums.
 constexpr int kTailBlock = 256;
 __global__ void __launch_bounds__(kTailBlock) k_fw_tail_small(LinkArgs a) {
@@ -2402,19 +2472,16 @@ __global__ void __launch_bounds__(kTailBlock) k_fw_tail_small(LinkArgs a) {
   const int passes = a.ls_mode == kLsExact ? kLsExactPasses : kLsPasses;
   for (int pass = 0; pass < passes; ++pass) {
     if (pass > 0 && !st.ls_pending) break;  // (uniform: written before the last barrier)
-    const int e0 = pass == 0 ? 1 : st.ls_next;
-    const double blo = pass == 0 ? 0.0 : st.ls_lo;
-    const double bhi = pass == 0 ? 1.0 : st.ls_hi;
+    const LsTry tr(st, a.ls_mode, pass);
     double acc[kNumSums];
 #pragma unroll
     for (int i = 0; i < kNumSums; ++i) acc[i] = 0.0;
-    for (int k = threadIdx.x; k < a.m; k += kTailBlock) ls_link(a, scen, off, cap, k, pass, e0, blo, bhi, acc);
+    for (int k = threadIdx.x; k < a.m; k += kTailBlock) ls_link(a, scen, off, cap, k, tr, acc);
     const double sum = block_sum16<kTailBlock>(acc, sh);
     if (threadIdx.x < kNumSums) tot[threadIdx.x] = sum;
     __syncthreads();
     if (threadIdx.x == 0)
-      ls_decide(st, tot, e0, pass, a.total_demand_s ? a.total_demand_s[scen] : a.total_demand,
-                a.ls_mode);
+      ls_decide(st, tot, tr, a.total_demand_s ? a.total_demand_s[scen] : a.total_demand);
     __syncthreads();
   }
   ls_fallback_block(a, scen, st, sh, &sh_found);
@@ -2692,8 +2759,8 @@ cudaError_t launch_ls_pass(const LinkArgs& a, int grid, int block, cudaStream_t 
   return cudaGetLastError();
 }
 
-cudaError_t launch_ls_fallback(const LinkArgs& a, cudaStream_t s) {
-  k_ls_fallback<<<dim3(1, a.num_scen), 1024, 0, s>>>(a);
+cudaError_t launch_ls_rest(const LinkArgs& a, cudaStream_t s) {
+  k_ls_rest<<<dim3(1, a.num_scen), kRestBlock, 0, s>>>(a);
   return cudaGetLastError();
 }
 

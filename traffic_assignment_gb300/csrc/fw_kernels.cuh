@@ -16,7 +16,7 @@
 namespace tapgpu {
 
 constexpr int kLsPerPass = 12;   // line-search candidates 2^-k evaluated per pass
-constexpr int kLsPasses = 5;     // passes captured per iteration (k up to 60)
+constexpr int kLsPasses = 5;     // passes of an iteration (k up to 60)
 constexpr int kLsMaxHalvings = 1000;  // tap/tap_functions.c:472
 constexpr int kNumSums = 4 + kLsPerPass;  // g0, vht, obj, g(1), g(2^-j) ...
 constexpr int kTraceCols = 8;    // obj, relgap, avg_excess, vht, lambda, gap, iter, g0
@@ -61,6 +61,7 @@ struct ScenState {
   double relgap, best_lb, obj, gap, lambda, vht, avg_excess, g0;
   double vht_end;  // VHT at the current x with the current costs
   double ls_lo, ls_hi, ls_glo, ls_ghi;  // exact line search: bracket of the root of g
+  double ls_root;  // and the estimate of the root that the next pass looks around
 };
 
 // line-search modes
@@ -68,7 +69,7 @@ enum : int {
   kLsReference = 0,  // largest 2^-k with g(2^-k) <= 0 (tap/tap_functions.c:469-507)
   kLsExact = 1,      // root of g on [0, 1] (differentiable: used by the adjoint)
 };
-constexpr int kLsExactPasses = 14;  // bracket shrinks 13x per pass
+constexpr int kLsExactPasses = 28;  // the bracket shrinks 13 times in every other one at least
 
 struct Demand {
   const int* od_ptr;            // [num_sources+1]
@@ -203,7 +204,7 @@ constexpr int kSmallLinkBlock = 64;
 // weights of the label-correction kernels' records from the current costs t
 cudaError_t launch_records(const LinkArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_ls_pass(const LinkArgs& a, int grid, int block, cudaStream_t s);
-cudaError_t launch_ls_fallback(const LinkArgs& a, cudaStream_t s);
+cudaError_t launch_ls_rest(const LinkArgs& a, cudaStream_t s);  // passes a.pass and on
 cudaError_t launch_step(const LinkArgs& a, int grid, int block, cudaStream_t s);
 // small networks (at most kSmallTail links): every line-search pass, the
 // fallback and the step in one launch (one block per scenario)

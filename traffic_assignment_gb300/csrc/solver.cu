@@ -875,12 +875,10 @@ int Ctx::enqueue_tail(int nscen) {
     return TAPGPU_OK;
   }
   TG_TRY(mark(2, true));
-  const int passes = ls_mode == kLsExact ? kLsExactPasses : kLsPasses;
-  for (int p = 0; p < passes; ++p) {
-    la.pass = p;
+  const int passes = grid_passes();
+  for (la.pass = 0; la.pass < passes; ++la.pass)
     TG_CUDA(launch_ls_pass(la, ls_grid(nscen), ls_block, stream));
-  }
-  TG_CUDA(launch_ls_fallback(la, stream));
+  TG_CUDA(launch_ls_rest(la, stream));
   TG_TRY(mark(2, false));
   TG_TRY(mark(3, true));
   TG_CUDA(launch_step(la, step_grid(nscen), ls_block, stream));
@@ -2254,11 +2252,9 @@ int tapgpu_profile_iteration(tapgpu_ctx* ctx, int reps, float* ms) {
     cudaEventRecord(ev[2], c->stream);
     }
     tapgpu::LinkArgs la = c->link_args(1);
-    for (int p = 0; p < tapgpu::kLsPasses; ++p) {
-      la.pass = p;
+    for (la.pass = 0; la.pass < c->grid_passes(); ++la.pass)
       tapgpu::launch_ls_pass(la, c->ls_grid(1), c->ls_block, c->stream);
-    }
-    tapgpu::launch_ls_fallback(la, c->stream);
+    tapgpu::launch_ls_rest(la, c->stream);
     cudaEventRecord(ev[3], c->stream);
     tapgpu::launch_step(la, c->step_grid(1), c->ls_block, c->stream);
     cudaEventRecord(ev[4], c->stream);

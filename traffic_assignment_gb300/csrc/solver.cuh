@@ -201,6 +201,9 @@ struct Ctx {
     const int want = (16 * num_sms + nscen - 1) / (nscen > 0 ? nscen : 1);
     return want < 1 ? 1 : (want > step_grid(nscen) ? step_grid(nscen) : want);
   }
+  // line-search passes over the whole grid (few open ones are left to k_ls_rest:
+  // steps below 2^-24, of small networks 2^-12; exact roots after six passes)
+  int grid_passes() const { return ls_mode == kLsExact ? 6 : (M <= kSmallNet ? 1 : 2); }
   // One scenario whose links make a few more blocks than there are SMs: one
   // block per SM, its share a little longer (40,000 links: 157 blocks gave five
   // SMs twice the FP64 work).
