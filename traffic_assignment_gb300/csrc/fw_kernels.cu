@@ -1224,6 +1224,17 @@ __global__ void __launch_bounds__(BLOCK, (1280 / BLOCK > 0 ? 1280 / BLOCK : 1)) 
   }
 }
 
+// A block's next task: off the work counter, or, without one, the block's own
+// (as many blocks as tasks: two round trips to the counter and the node that
+// clears it less, 5 us of a 40 us iteration on 24 nodes).
+__device__ __forceinline__ int next_task(const PathArgs& a, int round, int* sh_task) {
+  if (!a.counter) return round == 0 ? a.task_begin + static_cast<int>(blockIdx.x) : a.task_end;
+  __syncthreads();
+  if (threadIdx.x == 0) *sh_task = atomicAdd(a.counter, 1) + a.task_begin;
+  __syncthreads();
+  return *sh_task;
+}
+
 // ---------------------------------------------------------------------------
 // k_sssp_small: Bellman-Ford sweeps over an edge list held in shared memory
 // ---------------------------------------------------------------------------
@@ -1342,11 +1353,8 @@ __global__ void __launch_bounds__(kEdgeBlock) k_sssp_edges(PathArgs a) {
   }
   int staged = -1;  // scenario whose weights are in registers
 
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) sh_task = atomicAdd(a.counter, 1) + a.task_begin;
-    __syncthreads();
-    const int task = sh_task;
+  for (int round = 0;; ++round) {
+    const int task = next_task(a, round, &sh_task);
     if (task >= a.task_end) break;
     const int slot = task / a.num_sources;
     const int scen = a.scen_list ? a.scen_list[slot] : 0;
@@ -1447,11 +1455,8 @@ __global__ void __launch_bounds__(BLOCK, COMPACT ? (sizeof(T) == 4 ? 2048 : 1024
   unsigned short* par16 = reinterpret_cast<unsigned short*>(base + align16(8 * static_cast<size_t>(n1)));
   const int F = a.g.first_thru;
 
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) sh_task = atomicAdd(a.counter, 1) + a.task_begin;
-    __syncthreads();
-    const int task = sh_task;
+  for (int round = 0;; ++round) {
+    const int task = next_task(a, round, &sh_task);
     if (task >= a.task_end) break;
     const int slot = task / a.num_sources;
     const int scen = a.scen_list ? a.scen_list[slot] : 0;
@@ -2617,6 +2622,10 @@ size_t aon_smem_bytes(int n1, bool fp64, bool c64) {
   const size_t n = static_cast<size_t>(n1);
   if (aon_compact(n1, fp64) || (fp64 && c64)) return align16(align16(8 * n) + align16(2 * n));
   return align16(align16((fp64 ? 8 : 4) * n) + 2 * 4 * n);  // (FP32: 4-byte labels and totals)
+}
+
+bool sssp_own_tasks(int m, int variant, int block, bool smem) {
+  return sssp_edges(m, variant, block, smem);
 }
 
 int max_smem_optin(int device) {

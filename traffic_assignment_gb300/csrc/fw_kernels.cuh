@@ -101,7 +101,7 @@ struct PathArgs {
   int task_begin, task_end;     // task t: scenario scen_list[t / num_sources],
                                 //         source sources[t % num_sources]
   void* dist;                   // [(t - task_begin)][n1]
-  int* counter;                 // work counter, zero before launch
+  int* counter;                 // work counter, zero before launch (null: a block per task)
   int* err;                     // error bits
   int* err_info;                // [2]: origin, destination of a missing path
   int max_rounds;
@@ -190,6 +190,8 @@ constexpr int kSmallNet = 4096;
 // and step (above it the multi-block passes spread the FP64 work over SMs)
 constexpr int kSmallTail = 512;
 constexpr int kQueueSlots = 1024;  // ring slots of k_sssp_nfq
+// whether launch_sssp and launch_aon take a null counter (a block per task)
+bool sssp_own_tasks(int m, int variant, int block, bool smem);
 cudaError_t launch_sssp(const PathArgs& a, bool fp64, int grid, int block, bool smem,
                         int variant, cudaStream_t s);
 cudaError_t launch_aon(const PathArgs& a, bool fp64, int grid, int block, bool smem,

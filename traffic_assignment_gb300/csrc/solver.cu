@@ -830,13 +830,16 @@ int Ctx::enqueue_paths(int nscen, bool load, const uint2* e32p, const uint2* r32
     }
     const int ntask = static_cast<int>(t1 - t0);
     a.scratch_stride = static_cast<long long>(sssp_smem_bytes(n1, fp64, sssp_variant, M));
-    TG_CUDA(cudaMemsetAsync(counters, 0, 2 * sizeof(int), stream));
-    a.counter = counters;
+    // a block per task where the grids hold all of them
+    const bool own = sssp_own_tasks(M, sssp_variant, sssp_block, sssp_smem) && ntask <= sssp_grid;
+    const bool own_aon = ntask <= aon_grid;
+    if (!own || !own_aon) TG_CUDA(cudaMemsetAsync(counters, 0, 2 * sizeof(int), stream));
+    a.counter = own ? nullptr : counters;
     if (measuring) TG_TRY(mark(0, true));
     TG_CUDA(launch_sssp(a, fp64, std::min(sssp_grid, ntask), sssp_block, sssp_smem, sssp_variant,
                         stream));
     if (measuring) TG_TRY(mark(0, false));
-    a.counter = counters + 1;
+    a.counter = own_aon ? nullptr : counters + 1;
     a.scratch_stride = static_cast<long long>(aon_smem_bytes(n1, fp64, aon_c64));
     if (measuring) TG_TRY(mark(1, true));
     TG_CUDA(launch_aon(a, fp64, std::min(aon_grid, ntask), aon_block, aon_smem, stream));
@@ -1336,7 +1339,10 @@ static int equal_parts(int total, int cap) {
 static int iterate_until_done(Ctx* c, int S, int max_iters, std::vector<ScenState>& st) {
   // iterations per graph launch: enough to hide launch gaps, few enough that
   // finished scenarios do not linger
-  const int cap = c->opt.iters_per_launch > 0 ? c->opt.iters_per_launch : (S == 1 ? 8 : 4);
+  // (small networks: the wait and the state's copy after a launch cost 30 us)
+  const bool small = c->n1 <= kSmallNet && c->M <= kSmallNet;
+  const int cap = c->opt.iters_per_launch > 0 ? c->opt.iters_per_launch
+                                              : (S == 1 ? (small ? 16 : 8) : 4);
   const int per = equal_parts(max_iters, cap);
   std::vector<int> active;
   for (;;) {
@@ -2044,15 +2050,6 @@ int tapgpu_sssp(tapgpu_ctx* ctx, const double* weights, const int64_t* srcs, int
         }
       }
     }
-    cudaMemsetAsync(c->counters, 0, 2 * sizeof(int), c->stream);
-    a.counter = c->counters;
-    a.scratch_stride = static_cast<long long>(tapgpu::sssp_smem_bytes(n1, true, c->sssp_variant, c->M));
-    if (tapgpu::launch_sssp(a, true, grid, c->sssp_block, s_smem, c->sssp_variant, c->stream) !=
-        cudaSuccess) {
-      rc = TAPGPU_ERR_CUDA;
-      break;
-    }
-    a.counter = c->counters + 1;
     // FP64 labels: the 16-byte-per-node loading layout, whatever the context's
     const size_t abytes = tapgpu::aon_smem_bytes(n1, true);
     const bool a_smem = abytes + 1024 <= static_cast<size_t>(optin) && !c->opt.global_scratch;
@@ -2065,6 +2062,16 @@ int tapgpu_sssp(tapgpu_ctx* ctx, const double* weights, const int64_t* srcs, int
         break;
       }
     }
+    const bool own = tapgpu::sssp_own_tasks(c->M, c->sssp_variant, c->sssp_block, s_smem) && grid == ns;
+    if (!own || agrid < ns) cudaMemsetAsync(c->counters, 0, 2 * sizeof(int), c->stream);
+    a.counter = own ? nullptr : c->counters;
+    a.scratch_stride = static_cast<long long>(tapgpu::sssp_smem_bytes(n1, true, c->sssp_variant, c->M));
+    if (tapgpu::launch_sssp(a, true, grid, c->sssp_block, s_smem, c->sssp_variant, c->stream) !=
+        cudaSuccess) {
+      rc = TAPGPU_ERR_CUDA;
+      break;
+    }
+    a.counter = agrid == ns ? nullptr : c->counters + 1;
     a.scratch_stride = static_cast<long long>(abytes);
     if (tapgpu::launch_aon(a, true, agrid, c->aon_block, a_smem, c->stream) != cudaSuccess) {
       rc = TAPGPU_ERR_CUDA;
