@@ -2335,9 +2335,9 @@ __device__ void ls_fallback_block(const LinkArgs& a, int scen, ScenState& st, do
 }
 
 // The passes from a.pass on by one block per scenario, for a search that the
-// passes over the whole grid left open (steps below 2^-24, of small networks
-// below 2^-12), and the halvings beyond them.  Launches that find nothing to do
-// cost 2 us each: one for all of them instead of one per pass.
+// passes over the whole grid left open, and the halvings beyond them.  Launches
+// that find nothing to do cost 2 us each: one for all of them instead of one per
+// pass.
 constexpr int kRestBlock = 512;
 __global__ void __launch_bounds__(kRestBlock) k_ls_rest(LinkArgs a) {
   __shared__ double sh[kNumSums * (kRestBlock / 32)];
@@ -2502,29 +2502,9 @@ __global__ void __launch_bounds__(kTailBlock) k_fw_tail_small(LinkArgs a) {
   if (threadIdx.x == 0) step_finish(a, scen, st, it, lam, tp, acc[0]);
 }
 
-// Raise a kernel's dynamic shared-memory limit to the device maximum once, so
-// that launches inside a stream capture never change function attributes.
 template <typename Fn>
 cudaError_t allow_max_smem(Fn fn) {
-  // one flag per kernel (all path kernels share the same function type)
-  static std::mutex mu;
-  static std::set<std::pair<const void*, int>> done_set;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lock(mu);
-  const auto key = std::make_pair(reinterpret_cast<const void*>(fn), dev);
-  if (done_set.count(key)) return cudaSuccess;
-  cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, fn);
-  if (e != cudaSuccess) return e;
-  // the opt-in limit covers static and dynamic shared memory together
-  const int dyn = max_smem_optin(dev) - static_cast<int>(fa.sharedSizeBytes);
-  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
-  if (e == cudaSuccess)
-    done_set.insert(key);
-  else
-    cudaGetLastError();
-  return e;
+  return allow_max_smem_of(reinterpret_cast<const void*>(fn));
 }
 
 using PathKernel = void (*)(PathArgs);
@@ -2626,6 +2606,28 @@ size_t aon_smem_bytes(int n1, bool fp64, bool c64) {
 
 bool sssp_own_tasks(int m, int variant, int block, bool smem) {
   return sssp_edges(m, variant, block, smem);
+}
+
+cudaError_t allow_max_smem_of(const void* fn) {
+  // one flag per kernel and device
+  static std::mutex mu;
+  static std::set<std::pair<const void*, int>> done_set;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  const auto key = std::make_pair(fn, dev);
+  if (done_set.count(key)) return cudaSuccess;
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+  if (e != cudaSuccess) return e;
+  // the opt-in limit covers static and dynamic shared memory together
+  const int dyn = max_smem_optin(dev) - static_cast<int>(fa.sharedSizeBytes);
+  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
+  if (e == cudaSuccess)
+    done_set.insert(key);
+  else
+    cudaGetLastError();
+  return e;
 }
 
 int max_smem_optin(int device) {

@@ -190,6 +190,10 @@ constexpr int kSmallNet = 4096;
 // and step (above it the multi-block passes spread the FP64 work over SMs)
 constexpr int kSmallTail = 512;
 constexpr int kQueueSlots = 1024;  // ring slots of k_sssp_nfq
+// Raise a kernel's dynamic shared-memory limit to the device maximum once, so
+// that launches inside a stream capture, and those of other threads' contexts,
+// never change function attributes.
+cudaError_t allow_max_smem_of(const void* fn);
 // whether launch_sssp and launch_aon take a null counter (a block per task)
 bool sssp_own_tasks(int m, int variant, int block, bool smem);
 cudaError_t launch_sssp(const PathArgs& a, bool fp64, int grid, int block, bool smem,

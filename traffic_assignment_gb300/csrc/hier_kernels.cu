@@ -1514,9 +1514,8 @@ __global__ void __launch_bounds__(kElimBlock) k_hier_exponents(HierArgs a) {
 }
 
 template <typename Fn>
-cudaError_t max_smem(Fn fn, size_t bytes) {
-  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              static_cast<int>(bytes));
+cudaError_t max_smem(Fn fn) {
+  return allow_max_smem_of(reinterpret_cast<const void*>(fn));
 }
 
 // in clusters (1: none); early: see wait_for_previous
@@ -1546,7 +1545,7 @@ cudaError_t launch_with(Fn fn, dim3 grid, int block, size_t smem, int cluster, b
 }
 
 cudaError_t eliminate_t(const HierArgs& a, int num_levels, const int* tile_ptr, cudaStream_t s) {
-  cudaError_t e = max_smem(k_hier_mark, sizeof(MarkShared));
+  cudaError_t e = max_smem(k_hier_mark);
   if (e != cudaSuccess) return e;
   const int wb = (3 * a.h.arcs + 4 * kElimBlock - 1) / (4 * kElimBlock);
   k_hier_weights<<<dim3(wb, a.nslots), kElimBlock, 0, s>>>(a);
@@ -1566,7 +1565,7 @@ cudaError_t eliminate_t(const HierArgs& a, int num_levels, const int* tile_ptr, 
 cudaError_t climb_t(const HierArgs& a, cudaStream_t s) {
   const size_t per = hier_climb_smem(a.h.climb);
   const int warps = static_cast<int>(std::max<size_t>(1, std::min<size_t>(4, kHierMaxClimb / per)));
-  cudaError_t e = max_smem(k_hier_climb, per * warps);
+  cudaError_t e = max_smem(k_hier_climb);
   if (e != cudaSuccess) return e;
   const long long tasks = static_cast<long long>(a.nslots) * a.num_sources;
   k_hier_climb<<<static_cast<unsigned>((tasks + warps - 1) / warps), 32 * warps, per * warps, s>>>(a);
@@ -1576,7 +1575,7 @@ cudaError_t climb_t(const HierArgs& a, cudaStream_t s) {
 cudaError_t descend_t(const HierArgs& a, cudaStream_t s) {
   const size_t per = sizeof(Int) * static_cast<size_t>(a.h.climb);
   const int warps = static_cast<int>(std::max<size_t>(1, std::min<size_t>(4, kHierMaxClimb / per)));
-  cudaError_t e = max_smem(k_hier_descend, per * warps);
+  cudaError_t e = max_smem(k_hier_descend);
   if (e != cudaSuccess) return e;
   const long long tasks = static_cast<long long>(a.nslots) * a.num_sources;
   k_hier_descend<<<static_cast<unsigned>((tasks + warps - 1) / warps), 32 * warps, per * warps, s>>>(a);
@@ -1586,7 +1585,7 @@ cudaError_t descend_t(const HierArgs& a, cudaStream_t s) {
 template <int T>
 cudaError_t top_t(const HierArgs& a, int cluster, cudaStream_t s) {
   const size_t smem = sizeof(TopShared<T>) * (kTopBlock / 32);
-  cudaError_t e = max_smem(k_hier_top<T>, smem);
+  cudaError_t e = max_smem(k_hier_top<T>);
   if (e != cudaSuccess) return e;
   return launch_with(k_hier_top<T>, dim3(a.nslots * a.groups * cluster), kTopBlock, smem, cluster, false, s, a, cluster);
 }
@@ -1605,7 +1604,7 @@ cudaError_t sweep_t(const HierArgs& a, int num_sms, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   if (a.h.num_subs > 0) {
     const size_t smem = sizeof(SubShared) * kSubWarps;
-    if ((e = max_smem(k_hier_subs, smem)) != cudaSuccess) return e;
+    if ((e = max_smem(k_hier_subs)) != cudaSuccess) return e;
     const long long tasks = static_cast<long long>(cells) * a.h.num_subs;
     k_hier_subs<<<static_cast<unsigned>((tasks + kSubWarps - 1) / kSubWarps), kSubWarps * 32, smem, s>>>(a);
   }
