@@ -10,7 +10,7 @@ from scipy.sparse.csgraph import dijkstra
 
 from traffic_assignment_gb300 import Solver
 from traffic_assignment_gb300._capi import TapGpuError
-from traffic_assignment_gb300.synth import Demand, Network, Scenario
+from traffic_assignment_gb300.synth import Demand, Network, Scenario, make_workload
 
 pytestmark = pytest.mark.gpu
 
@@ -218,3 +218,25 @@ def test_paths_change_with_the_batch(built_lib):
         s.solve_scenarios(scen, max_iters=2)
         s.run_iterations(3)
         np.testing.assert_array_equal(many, s.flows_batch()[0])
+
+
+def test_one_loading_at_given_costs(built_lib):
+    """aon() of a context whose single loadings pay, at the free-flow costs'
+    scale, far from it (the exponent is found anew) and in between solves: the
+    label-correction kernels' volumes."""
+    net, dem = make_workload("grid10k")
+    rng = np.random.default_rng(17)
+    w = net.fft * rng.lognormal(0.0, 0.5, net.num_links)
+    out = []
+    for variant in ("default", "nearfar_queue"):
+        with Solver(net, dem, precision="fp64", sssp_variant=variant) as s:
+            y, on = _on_hierarchy(s, lambda: [s.aon(w * f) for f in (1.0, 2.0 ** 12, 2.0 ** -30)])
+            assert on == (variant == "default")
+            y.append(s.aon(w * 2.0 ** 40))  # (beyond the exponents that are tried)
+            s.solve(max_iters=2)
+            y += [s.aon(w), s.flows()[0]]
+            out.append(y)
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    for y in out[0][1:4]:  # a power of two changes no path
+        np.testing.assert_array_equal(y, out[0][0])

@@ -337,7 +337,7 @@ bool Ctx::hier_pays(int nscen, int levels, double relaxations, int arcs) const {
 
 // The path kernels of the next iterations of nscen scenarios, and their buffers.
 int Ctx::choose_paths(int nscen) {
-  bool on = hier && hier_pays(nscen, static_cast<int>(h_tile_ptr.size()) - 1, hier_relaxations, hg.arcs);
+  bool on = hier && hier_pays(nscen);
   if (on && hier_cap < nscen) {
     if (gexec) cudaGraphExecDestroy(gexec);
     gexec = nullptr;
@@ -639,6 +639,26 @@ int Ctx::ensure_hier(int S) {
 // Shortest paths and loading of the first nscen entries of scen_list at link
 // costs cost[scenario * stride + link], into yfx.
 int Ctx::enqueue_hier(int nscen, const double* cost, long long stride, cudaEvent_t between) {
+  HierArgs a = hier_args(cost, stride);
+  for (int s0 = 0; s0 < nscen; s0 += hier_slots) {
+    a.slot0 = s0;
+    a.nslots = std::min(hier_slots, nscen - s0);
+    if (measuring) TG_TRY(mark(0, true));
+    const int levels = static_cast<int>(h_tile_ptr.size()) - 1;
+    TG_CUDA(launch_hier_eliminate(a, levels, h_tile_ptr.data(), stream));
+    TG_CUDA(launch_hier_climb(a, stream));
+    TG_CUDA(launch_hier_sweep(a, num_sms, stream));
+    if (measuring) TG_TRY(mark(0, false));
+    if (between) TG_CUDA(cudaEventRecord(between, stream));
+    if (measuring) TG_TRY(mark(1, true));
+    TG_CUDA(launch_hier_load(a, num_sms, stream));
+    if (measuring) TG_TRY(mark(1, false));
+    count_launches(levels + 24);
+  }
+  return TAPGPU_OK;
+}
+
+HierArgs Ctx::hier_args(const double* cost, long long stride) const {
   HierArgs a;
   std::memset(&a, 0, sizeof(a));
   a.h = hg;
@@ -671,20 +691,46 @@ int Ctx::enqueue_hier(int nscen, const double* cost, long long stride, cudaEvent
   a.list = h_list;
   a.list_n = h_list_n;
   a.y_fx = yfx;
-  for (int s0 = 0; s0 < nscen; s0 += hier_slots) {
-    a.slot0 = s0;
-    a.nslots = std::min(hier_slots, nscen - s0);
-    if (measuring) TG_TRY(mark(0, true));
+  return a;
+}
+
+constexpr int kHierRetries = 4;
+constexpr int kHierRetryBits = 5;
+
+// One loading of the base demand at the costs of an API call (api_w64) into
+// api_yfx, with a state of its own.  *loaded stays false where the labels do
+// not fit after kHierRetries exponents: the label-correction kernels' case.
+int Ctx::hier_load_api(bool* loaded) {
+  HierArgs a = hier_args(api_w64, 0);
+  a.scen_list = nullptr;
+  a.absent = nullptr;
+  a.dest_dem = h_dem;
+  a.dest_stride = 0;
+  a.y_fx = api_yfx;
+  a.nslots = 1;
+  if (!api_state) TG_TRY(alloc_n(&api_state, 1));
+  a.state = api_state;
+  ScenState st;
+  std::memset(&st, 0, sizeof(st));
+  st.u_exp = u_exp0;
+  for (int tries = 0; tries <= kHierRetries; ++tries) {
+    TG_CUDA(cudaMemcpyAsync(api_state, &st, sizeof(st), cudaMemcpyHostToDevice, stream));
     const int levels = static_cast<int>(h_tile_ptr.size()) - 1;
     TG_CUDA(launch_hier_eliminate(a, levels, h_tile_ptr.data(), stream));
     TG_CUDA(launch_hier_climb(a, stream));
     TG_CUDA(launch_hier_sweep(a, num_sms, stream));
-    if (measuring) TG_TRY(mark(0, false));
-    if (between) TG_CUDA(cudaEventRecord(between, stream));
-    if (measuring) TG_TRY(mark(1, true));
     TG_CUDA(launch_hier_load(a, num_sms, stream));
-    if (measuring) TG_TRY(mark(1, false));
-    count_launches(levels + 24);
+    TG_CUDA(cudaStreamSynchronize(stream));
+    TG_CUDA(cudaMemcpy(&st, api_state, sizeof(st), cudaMemcpyDeviceToHost));
+    if (!st.done) {
+      *loaded = true;
+      return TAPGPU_OK;
+    }
+    if (st.done == kPaused) st.u_exp -= kHierRetryBits;
+    st.done = 0;
+    st.maxlab = 0;
+    TG_CUDA(cudaMemsetAsync(h_flow, 0, static_cast<size_t>(hier_slots) * 3 * hg.arcs *
+                                           sizeof(unsigned long long), stream));
   }
   return TAPGPU_OK;
 }
@@ -693,9 +739,6 @@ int Ctx::enqueue_hier(int nscen, const double* cost, long long stride, cudaEvent
 // exponent (those that used too little of it have their new one); one that
 // does so repeatedly takes this iteration with the label-correction kernels,
 // which also report a missing path.
-constexpr int kHierRetries = 4;
-constexpr int kHierRetryBits = 5;
-
 int Ctx::resume_paused(int S, std::vector<ScenState>& st) {
   if (!hier_on) return TAPGPU_OK;
   std::vector<int> legacy;
@@ -2114,9 +2157,15 @@ int tapgpu_aon(tapgpu_ctx* ctx, const double* weights, double* volume) {
   TG_TRY(to_device_weights(c, weights, w));
   TG_CUDA(cudaMemsetAsync(c->api_yfx, 0, sizeof(unsigned long long) * c->M, c->stream));
   TG_CUDA(cudaMemsetAsync(c->err, 0, sizeof(int), c->stream));
+  bool loaded = false;
+  if (c->hier && c->hier_cap >= 1 && c->hier_pays(1)) {
+    TG_TRY(c->hier_load_api(&loaded));
+    if (!loaded)
+      TG_CUDA(cudaMemsetAsync(c->api_yfx, 0, sizeof(unsigned long long) * c->M, c->stream));
+  }
   const double solver_delta = c->nf_delta;
   c->nf_delta = c->api_nf_delta;
-  const int rc = c->enqueue_paths(1, true, c->fp64 ? nullptr : c->api_e32,
+  const int rc = loaded ? TAPGPU_OK : c->enqueue_paths(1, true, c->fp64 ? nullptr : c->api_e32,
                                   c->fp64 ? nullptr : c->api_r32, c->fp64 ? c->api_w64 : nullptr,
                                   c->api_yfx, false);
   c->nf_delta = solver_delta;

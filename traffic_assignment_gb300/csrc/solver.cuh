@@ -139,6 +139,7 @@ struct Ctx {
   // otherwise, and for a scenario whose labels leave the integers' range
   bool hier = false;             // its plan is in place
   bool hier_on = false;          // the iterations run on it (choose_paths)
+  ScenState* api_state = nullptr;  // of a loading through the API
   int hier_cap = 0;              // scenarios that its buffers were made for
   HierGraph hg{};
   double hier_relaxations = 0;
@@ -251,9 +252,14 @@ struct Ctx {
   void release_hier();
   int ensure_hier(int S);
   bool hier_pays(int nscen, int levels, double relaxations, int arcs) const;
+  bool hier_pays(int nscen) const {
+    return hier_pays(nscen, static_cast<int>(h_tile_ptr.size()) - 1, hier_relaxations, hg.arcs);
+  }
   int choose_paths(int nscen);
   int ensure_legacy(int S);
   int enqueue_hier(int nscen, const double* cost, long long stride, cudaEvent_t between = nullptr);
+  HierArgs hier_args(const double* cost, long long stride) const;
+  int hier_load_api(bool* loaded);
   int begin_paths(int nscen);
   int set_active(const std::vector<int>& active);
   int resume_paused(int S, std::vector<ScenState>& st);
