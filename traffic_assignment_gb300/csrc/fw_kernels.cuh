@@ -182,7 +182,7 @@ enum : int {
   kSsspNearFar = 3, // asynchronous near set below a rising threshold (k_sssp_nf)
   kSsspNearFarQueue = 4,  // near-far with a FIFO ring of near nodes (k_sssp_nfq)
   kSsspNearFarQueueWide = 5,  // the same with 32-bit ring entries (chosen above 65535 nodes)
-  kSsspSmall = 6,   // Bellman-Ford sweeps over the edge list in shared memory (k_sssp_small;
+  kSsspSmall = 6,   // Bellman-Ford sweeps over the edge list (k_sssp_edges, k_sssp_small;
                     // chosen for networks of at most kSmallNet nodes and links)
 };
 constexpr int kSmallNet = 4096;
