@@ -1319,7 +1319,6 @@ static int create_impl(const tapgpu_network* net, const tapgpu_demand* dem,
 
   TG_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   TG_TRY(c->plan_launches());
-  TG_TRY(c->hier_plan(builder.wait(), odest, optr, odem));
   TG_TRY(c->alloc_n(&c->counters, 2));
   TG_TRY(c->alloc_n(&c->err, 1));
   TG_TRY(c->alloc_n(&c->err_info, 2));
@@ -1341,9 +1340,9 @@ static int create_impl(const tapgpu_network* net, const tapgpu_demand* dem,
   TG_TRY(c->alloc_n(&c->api_w64, M));
   TG_TRY(c->alloc_n(&c->api_yfx, M));
   TG_TRY(c->ensure_scenarios(1));
+  TG_CUDA(cudaMemcpy(c->cap, c->h_cap.data(), sizeof(double) * M, cudaMemcpyHostToDevice));
+  TG_TRY(c->hier_plan(builder.wait(), odest, optr, odem));
   TG_TRY(c->choose_paths(1));
-  std::vector<double> capv(c->h_cap);
-  TG_CUDA(cudaMemcpy(c->cap, capv.data(), sizeof(double) * M, cudaMemcpyHostToDevice));
   *out = guard.release();
   return TAPGPU_OK;
 }
