@@ -1327,6 +1327,7 @@ __global__ void k_hier_descend(HierArgs a) {
           f[t] += y;
         }
       }
+      __syncwarp();  // (the next row may add to the same slot; shuffles do not order memory)
     }
     __syncwarp();
   }
