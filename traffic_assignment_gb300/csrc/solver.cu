@@ -260,7 +260,25 @@ LinkArgs Ctx::link_args(int nscen, bool records) const {
 
 int Ctx::ensure_scenarios(int S) {
   if (S <= S_cap) return TAPGPU_OK;
-  // release the old per-scenario arrays
+  release_scenarios();
+  const int rc = alloc_scenarios(S);
+  if (rc != TAPGPU_OK) {
+    release_scenarios();
+    return rc;
+  }
+  S_cap = S;  // (last: a call after one that found no memory allocates again)
+  return TAPGPU_OK;
+}
+
+// The per-scenario arrays, and the captured launches that hold their addresses.
+void Ctx::release_scenarios() {
+  S_cap = 0;
+  if (gexec) {
+    cudaGraphExecDestroy(gexec);
+    gexec = nullptr;
+  }
+  g_nscen = -1;
+  h_scen_list.clear();
   void* olds[] = {cap, x, t, d, dtdx, yfx, e32, r32, e4, r4, r4d, w64, state, partials, arrive,
                   trace, scen_list, x_hist, d_hist, lam_hist};
   for (void* p : olds) free_owned(this, p);
@@ -278,13 +296,15 @@ int Ctx::ensure_scenarios(int S) {
   trace = nullptr;
   scen_list = nullptr;
   x_hist = d_hist = lam_hist = nullptr;
+}
+
+int Ctx::alloc_scenarios(int S) {
   const size_t sm = static_cast<size_t>(S) * M;
   TG_TRY(alloc_n(&cap, sm));
   TG_TRY(alloc_n(&x, sm));
   TG_TRY(alloc_n(&t, sm));
   TG_TRY(alloc_n(&d, sm));
   TG_TRY(alloc_n(&yfx, sm));
-  S_cap = S;
   if (opt.record_tape) TG_TRY(alloc_n(&dtdx, sm));
   TG_TRY(alloc_n(&state, static_cast<size_t>(S)));
   TG_TRY(alloc_n(&partials, static_cast<size_t>(S) * std::max(link_grid, ls_link_grid) * kNumSums));
@@ -293,7 +313,6 @@ int Ctx::ensure_scenarios(int S) {
   trace_cap = S == 1 ? 100000 : 4096;
   TG_TRY(alloc_n(&trace, static_cast<size_t>(S) * trace_cap * kTraceCols));
   TG_TRY(alloc_n(&scen_list, static_cast<size_t>(S)));
-  h_scen_list.clear();
   if (opt.record_tape && opt.tape_capacity > 0) {
     hist_cap = opt.tape_capacity;
     ckpt_every = opt.tape_checkpoint > 0
@@ -303,11 +322,6 @@ int Ctx::ensure_scenarios(int S) {
     TG_TRY(alloc_n(&d_hist, sm * hist_cap));
     TG_TRY(alloc_n(&lam_hist, static_cast<size_t>(S) * hist_cap));
   }
-  if (gexec) {
-    cudaGraphExecDestroy(gexec);
-    gexec = nullptr;
-  }
-  g_nscen = -1;
   return TAPGPU_OK;
 }
 
@@ -1471,6 +1485,7 @@ int tapgpu_set_capacity(tapgpu_ctx* ctx, const double* capacity) {
     c->h_cap[k] = v > 0 ? v : min_cap;
   }
   c->base_dirty = true;
+  if (!c->S_cap) return TAPGPU_OK;  // (no arrays after a failed allocation: the next solve copies it)
   TG_CUDA(cudaSetDevice(c->device));
   TG_CUDA(cudaMemcpy(c->cap, c->h_cap.data(), sizeof(double) * c->M, cudaMemcpyHostToDevice));
   return TAPGPU_OK;
@@ -1509,6 +1524,10 @@ int tapgpu_solve_begin(tapgpu_ctx* ctx, int max_iters, double target_relgap, con
 int tapgpu_solve_advance(tapgpu_ctx* ctx, int max_new_iters, int* done, tapgpu_result* res) {
   if (!ctx || max_new_iters < 1) return TAPGPU_ERR_ARG;
   Ctx* c = ctx->c;
+  if (!c->S_cap) {
+    tapgpu::set_message("no solve to go on with");
+    return TAPGPU_ERR_ARG;
+  }
   TG_CUDA(cudaSetDevice(c->device));
   std::vector<tapgpu::ScenState> st;
   TG_TRY(c->read_states(1, st));
@@ -2183,6 +2202,10 @@ void* tapgpu_stream(tapgpu_ctx* ctx) { return ctx ? ctx->c->stream : nullptr; }
 int tapgpu_run_iterations(tapgpu_ctx* ctx, int iters) {
   if (!ctx || iters < 1) return TAPGPU_ERR_ARG;
   Ctx* c = ctx->c;
+  if (!c->S_cap) {
+    tapgpu::set_message("no solve to go on with");
+    return TAPGPU_ERR_ARG;
+  }
   TG_CUDA(cudaSetDevice(c->device));
   const int S = c->last_nscen;
   std::vector<tapgpu::ScenState> st;
@@ -2267,6 +2290,10 @@ int tapgpu_get_timing(tapgpu_ctx* ctx, double* ms, int64_t* counts, int64_t* ker
 int tapgpu_profile_iteration(tapgpu_ctx* ctx, int reps, float* ms) {
   if (!ctx || !ms || reps < 1) return TAPGPU_ERR_ARG;
   Ctx* c = ctx->c;
+  if (!c->S_cap) {
+    tapgpu::set_message("no solve to go on with");
+    return TAPGPU_ERR_ARG;
+  }
   TG_CUDA(cudaSetDevice(c->device));
   std::vector<tapgpu::ScenState> st;
   TG_TRY(c->read_states(1, st));

@@ -225,6 +225,8 @@ struct Ctx {
     return alloc(reinterpret_cast<void**>(p), n * sizeof(T));
   }
   int ensure_scenarios(int S);
+  int alloc_scenarios(int S);
+  void release_scenarios();
   int plan_launches();
 
   Graph graph() const;
