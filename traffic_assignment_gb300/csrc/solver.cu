@@ -279,17 +279,12 @@ void Ctx::release_scenarios() {
   }
   g_nscen = -1;
   h_scen_list.clear();
-  void* olds[] = {cap, x, t, d, dtdx, yfx, e32, r32, e4, r4, r4d, w64, state, partials, arrive,
-                  trace, scen_list, x_hist, d_hist, lam_hist};
+  release_records();
+  void* olds[] = {cap, x, t, d, dtdx, yfx, state, partials, arrive, trace, scen_list, x_hist, d_hist,
+                  lam_hist};
   for (void* p : olds) free_owned(this, p);
   cap = x = t = d = dtdx = nullptr;
   yfx = nullptr;
-  e32 = nullptr;
-  e4 = nullptr;
-  r4 = nullptr;
-  r4d = nullptr;
-  r32 = nullptr;
-  w64 = nullptr;
   state = nullptr;
   partials = nullptr;
   arrive = nullptr;
@@ -361,7 +356,13 @@ int Ctx::choose_paths(int nscen) {
       on = false;
     }
   }
-  if (!on) TG_TRY(ensure_legacy(S_cap));
+  if (!on) {
+    const int rc = ensure_legacy(S_cap);
+    if (rc != TAPGPU_OK) {  // (the next call starts from its own number of scenarios)
+      release_scenarios();
+      return rc;
+    }
+  }
   if (on != hier_on && gexec) {
     cudaGraphExecDestroy(gexec);
     gexec = nullptr;
@@ -372,40 +373,67 @@ int Ctx::choose_paths(int nscen) {
 
 // The weight records and the label buffer of the label-correction kernels.
 int Ctx::ensure_legacy(int S) {
-  if (fp64 ? w64 != nullptr : e32 != nullptr) return TAPGPU_OK;
-  const size_t sm = static_cast<size_t>(S) * M;
-  if (fp64) {
-    TG_TRY(alloc_n(&w64, sm));
-    // slots beyond a node's in-links keep an infinite weight: never tight
-    const size_t s4 = static_cast<size_t>(S) * n1 * 4;
-    TG_TRY(alloc_n(&r4d, s4));
-    TG_CUDA(launch_fill_records4(r4d, s4, make_uint4(0u, 0u, 0u, 0x7ff00000u), 2 * num_sms, stream));
-  } else
-  {
-    TG_TRY(alloc_n(&e32, sm));
-    TG_TRY(alloc_n(&r32, sm));
-    const size_t s4 = static_cast<size_t>(S) * n1 * 4;
-    TG_TRY(alloc_n(&e4, s4));
-    TG_CUDA(cudaMemset(e4, 0, sizeof(uint2) * s4));
-    if (rev4) {
-      // slots beyond a node's in-links keep an infinite weight: never tight
-      TG_TRY(alloc_n(&r4, s4));
-      TG_CUDA(launch_fill_records(r4, s4, make_uint2(0u, 0x7f800000u), 2 * num_sms, stream));
-    }
+  if (records_ready) return TAPGPU_OK;
+  const int rc = alloc_records(S);
+  if (rc != TAPGPU_OK) {
+    release_records();
+    return rc;
   }
   // Unless the caller fixed the chunk, the label buffer grows to hold a whole
   // batch's tasks (up to 16 GiB), so that an iteration runs one shortest-path
   // and one loading launch instead of one per chunk, each with its tail.
-  if (opt.chunk_tasks <= 0 && dist) {
-    const int64_t tb = static_cast<int64_t>(n1) * (fp64 ? 8 : 4);
+  const int64_t tb = static_cast<int64_t>(n1) * (fp64 ? 8 : 4);
+  if (opt.chunk_tasks <= 0) {
     const int64_t want = std::min<int64_t>(std::max<int64_t>(1, (int64_t(16) << 30) / tb),
                                            static_cast<int64_t>(S) * std::max(Z, 1));
     if (want > dist_tasks) {
       free_owned(this, dist);
       dist = nullptr;
-      TG_TRY(alloc(&dist, static_cast<size_t>(tb) * static_cast<size_t>(want)));
-      dist_tasks = want;
+      if (alloc(&dist, static_cast<size_t>(tb) * static_cast<size_t>(want)) == TAPGPU_OK)
+        dist_tasks = want;
     }
+  }
+  const int held = ensure_labels();  // (no room for the larger one: by chunks of the first size)
+  if (held != TAPGPU_OK) {
+    release_records();
+    return held;
+  }
+  records_ready = true;  // (last: a call after one that found no memory allocates again)
+  return TAPGPU_OK;
+}
+
+// The label buffer of dist_tasks tasks.
+int Ctx::ensure_labels() {
+  if (dist) return TAPGPU_OK;
+  return alloc(&dist, static_cast<size_t>(n1) * (fp64 ? 8 : 4) * static_cast<size_t>(dist_tasks));
+}
+
+void Ctx::release_records() {
+  records_ready = false;
+  void* olds[] = {e32, r32, e4, r4, r4d, w64};
+  for (void* p : olds) free_owned(this, p);
+  e32 = r32 = e4 = r4 = nullptr;
+  r4d = nullptr;
+  w64 = nullptr;
+}
+
+int Ctx::alloc_records(int S) {
+  const size_t sm = static_cast<size_t>(S) * M, s4 = static_cast<size_t>(S) * n1 * 4;
+  if (fp64) {
+    TG_TRY(alloc_n(&w64, sm));
+    // slots beyond a node's in-links keep an infinite weight: never tight
+    TG_TRY(alloc_n(&r4d, s4));
+    TG_CUDA(launch_fill_records4(r4d, s4, make_uint4(0u, 0u, 0u, 0x7ff00000u), 2 * num_sms, stream));
+    return TAPGPU_OK;
+  }
+  TG_TRY(alloc_n(&e32, sm));
+  TG_TRY(alloc_n(&r32, sm));
+  TG_TRY(alloc_n(&e4, s4));
+  TG_CUDA(cudaMemsetAsync(e4, 0, sizeof(uint2) * s4, stream));
+  if (rev4) {
+    // slots beyond a node's in-links keep an infinite weight: never tight
+    TG_TRY(alloc_n(&r4, s4));
+    TG_CUDA(launch_fill_records(r4, s4, make_uint2(0u, 0x7f800000u), 2 * num_sms, stream));
   }
   return TAPGPU_OK;
 }
@@ -1346,7 +1374,7 @@ static int create_impl(const tapgpu_network* net, const tapgpu_demand* dem,
                                       : std::max<int64_t>(1, (int64_t(2) << 30) / static_cast<int64_t>(tb));
   chunk = std::max<int64_t>(1, std::min<int64_t>(chunk, 1 << 30));
   c->dist_tasks = std::min<int64_t>(chunk, std::max<int64_t>(Z, 1) * 4096);
-  TG_TRY(c->alloc(&c->dist, tb * c->dist_tasks));
+  TG_TRY(c->ensure_labels());
   TG_TRY(c->alloc_n(&c->api_e32, M));
   TG_TRY(c->alloc_n(&c->api_e4, static_cast<size_t>(n1) * 4));
   TG_CUDA(cudaMemset(c->api_e4, 0, sizeof(uint2) * static_cast<size_t>(n1) * 4));
@@ -1524,7 +1552,7 @@ int tapgpu_solve_begin(tapgpu_ctx* ctx, int max_iters, double target_relgap, con
 int tapgpu_solve_advance(tapgpu_ctx* ctx, int max_new_iters, int* done, tapgpu_result* res) {
   if (!ctx || max_new_iters < 1) return TAPGPU_ERR_ARG;
   Ctx* c = ctx->c;
-  if (!c->S_cap) {
+  if (!c->can_iterate()) {
     tapgpu::set_message("no solve to go on with");
     return TAPGPU_ERR_ARG;
   }
@@ -2048,6 +2076,7 @@ int tapgpu_sssp(tapgpu_ctx* ctx, const double* weights, const int64_t* srcs, int
   std::vector<double> w;
   TG_TRY(to_device_weights(c, weights, w));
   const int n1 = c->n1;
+  TG_TRY(c->ensure_labels());
   // FP64 labels: a FP32 context's label buffer holds half as many sources
   const int64_t chunk = c->fp64 ? c->dist_tasks : std::max<int64_t>(1, c->dist_tasks / 2);
   const int64_t rows = std::max<int64_t>(1, std::min(chunk, num_sources));
@@ -2181,6 +2210,7 @@ int tapgpu_aon(tapgpu_ctx* ctx, const double* weights, double* volume) {
     if (!loaded)
       TG_CUDA(cudaMemsetAsync(c->api_yfx, 0, sizeof(unsigned long long) * c->M, c->stream));
   }
+  if (!loaded) TG_TRY(c->ensure_labels());
   const double solver_delta = c->nf_delta;
   c->nf_delta = c->api_nf_delta;
   const int rc = loaded ? TAPGPU_OK : c->enqueue_paths(1, true, c->fp64 ? nullptr : c->api_e32,
@@ -2202,7 +2232,7 @@ void* tapgpu_stream(tapgpu_ctx* ctx) { return ctx ? ctx->c->stream : nullptr; }
 int tapgpu_run_iterations(tapgpu_ctx* ctx, int iters) {
   if (!ctx || iters < 1) return TAPGPU_ERR_ARG;
   Ctx* c = ctx->c;
-  if (!c->S_cap) {
+  if (!c->can_iterate()) {
     tapgpu::set_message("no solve to go on with");
     return TAPGPU_ERR_ARG;
   }
@@ -2290,7 +2320,7 @@ int tapgpu_get_timing(tapgpu_ctx* ctx, double* ms, int64_t* counts, int64_t* ker
 int tapgpu_profile_iteration(tapgpu_ctx* ctx, int reps, float* ms) {
   if (!ctx || !ms || reps < 1) return TAPGPU_ERR_ARG;
   Ctx* c = ctx->c;
-  if (!c->S_cap) {
+  if (!c->can_iterate()) {
     tapgpu::set_message("no solve to go on with");
     return TAPGPU_ERR_ARG;
   }

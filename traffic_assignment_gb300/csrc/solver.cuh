@@ -97,6 +97,7 @@ struct Ctx {
   int* rpos = nullptr;   // reverse-star slot of each link
   std::vector<int> h_rpos;
   double* w64 = nullptr;
+  bool records_ready = false;  // e32 .. r4 or w64, r4d of S_cap scenarios are there
   ScenState* state = nullptr;
   double* partials = nullptr;
   unsigned* arrive = nullptr;
@@ -259,6 +260,11 @@ struct Ctx {
   }
   int choose_paths(int nscen);
   int ensure_legacy(int S);
+  int alloc_records(int S);
+  void release_records();
+  int ensure_labels();
+  // the arrays of the last solve are there
+  bool can_iterate() const { return S_cap > 0 && (hier_on || records_ready); }
   int enqueue_hier(int nscen, const double* cost, long long stride, cudaEvent_t between = nullptr);
   HierArgs hier_args(const double* cost, long long stride) const;
   int hier_load_api(bool* loaded);
