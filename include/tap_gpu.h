@@ -394,6 +394,12 @@ int tapgpu_set_scenario_links(tapgpu_ctx *ctx, int num_scen, const int64_t *edit
  * iterations on the elimination hierarchy leave them as they are.) */
 int tapgpu_get_path_stats(tapgpu_ctx *ctx, int64_t *out);
 
+/* Bound in bytes of the elimination hierarchy's per-scenario buffers (FP64
+ * iterations; default 24 GiB, which bytes <= 0 restores): of a batch that needs
+ * more, scenarios take turns in what the bound holds, at least one at a time.
+ * Gives the present buffers back; the next solve makes its own. */
+int tapgpu_set_hierarchy_limit(tapgpu_ctx *ctx, int64_t bytes);
+
 /* No counterpart in the reference.  All-origins FP64 shortest-path labels for
  * callers that cannot let a library allocate device memory (their own pool
  * owns the HBM, or a cudaMalloc/cudaFree and the device synchronisation it

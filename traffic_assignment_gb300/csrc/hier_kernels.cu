@@ -24,8 +24,9 @@
 // labels are equal exactly, and comparisons against shortcut sums need no
 // tolerance.  The exponent of a scenario follows its largest label, which gets
 // kBits + 1 bits the next time.  A label that leaves the range pauses the
-// scenario (done = kPaused), and so does a largest label of less than kMinBits
-// + 1 bits (kCoarse): the host repeats the iteration at another exponent.  So a
+// scenario (done = kPausing, at the end of the loading kPaused), and so does a
+// largest label of less than kMinBits + 1 bits (kCoarse): the host repeats the
+// iteration at another exponent.  So a
 // link's rounding is at most 2^-54 of the largest label, that of an FP64 sum
 // up to 2^-53 of the sum at every link.
 //
@@ -862,7 +863,7 @@ struct DemandAt {
   }
   // by whole warps
   __device__ __forceinline__ void report(ScenState& st) {
-    if (out_of_range) st.done = kPaused;
+    if (out_of_range) st.done = kPausing;
     Int x = largest;
 #pragma unroll
     for (int z = 16; z >= 1; z >>= 1) {
@@ -1163,14 +1164,16 @@ __global__ void __launch_bounds__(kSubWarps * 32) k_hier_subs(HierArgs a) {
 // Volumes of the top chunks of one scenario and group per cluster, from the
 // lowest level; each row's volume goes to the upper neighbour that gave its
 // label.  (Runs for a scenario that paused in this iteration too: it leaves
-// the volumes zero.)
+// the volumes zero.  One that paused before has no labels here: the slot may
+// hold another scenario's.)
 template <int N, bool AHEAD>
 __global__ void __launch_bounds__(kTopBlock, AHEAD ? 1 : 4) k_hier_volumes(HierArgs a, int cluster) {
   const HierGraph& h = a.h;
   const int cell = blockIdx.x / cluster;
   const int slot = cell / a.groups, grp = cell - slot * a.groups;
   const int scen = a.scen_list ? a.scen_list[a.slot0 + slot] : 0;
-  if (a.state[scen].done == 1) return;
+  const int done = a.state[scen].done;
+  if (done && done != kPausing) return;
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x % cluster) * (kTopBlock / 32) + (threadIdx.x >> 5);
   const int warps = cluster * (kTopBlock / 32);
@@ -1344,10 +1347,18 @@ constexpr int kCollect = 4;  // arcs per thread
 __global__ void __launch_bounds__(kElimBlock) k_hier_collect(HierArgs a) {
   const int slot = blockIdx.y;
   const int scen = a.scen_list ? a.scen_list[a.slot0 + slot] : 0;
-  if (a.state[scen].done) return;
+  const int done = a.state[scen].done;
+  if (done && done != kPausing) return;
   const int arcs3 = 3 * a.h.arcs, lane = threadIdx.x & 31;
   const unsigned long long* mid = a.mid + static_cast<size_t>(slot) * arcs3;
   unsigned long long* flow = a.flow + static_cast<size_t>(slot) * arcs3;
+  if (done) {  // paused: what the sweep added is for nobody
+    for (int z = 0; z < kCollect; ++z) {
+      const int s = blockIdx.x * (kCollect * kElimBlock) + z * kElimBlock + threadIdx.x;
+      if (s < arcs3) flow[s] = 0ull;
+    }
+    return;
+  }
   int* list = a.list + static_cast<size_t>(slot) * 2 * arcs3;
   __shared__ int count, base;
   if (threadIdx.x == 0) count = 0;
@@ -1506,6 +1517,7 @@ __global__ void __launch_bounds__(kElimBlock) k_hier_exponents(HierArgs a) {
   const int slot = blockIdx.x * kElimBlock + threadIdx.x;
   if (slot >= a.nslots) return;
   ScenState& st = a.state[a.scen_list ? a.scen_list[a.slot0 + slot] : 0];
+  if (st.done == kPausing) st.done = kPaused;
   if (st.done || !st.maxlab) return;
   const int top = 63 - __clzll(static_cast<long long>(st.maxlab));
   const int u_exp = max(-kMaxExp, min(kMaxExp, st.u_exp + kBits - top));

@@ -7,8 +7,9 @@
 namespace tapgpu {
 
 // ScenState::done: labels left the integer range, or used too little of it
-// (see hier_kernels.cu)
-constexpr int kPaused = 2, kCoarse = 3;
+// (see hier_kernels.cu); kPausing: left it in the iteration under way, whose
+// loading empties the scenario's buffers and then makes it kPaused
+constexpr int kPaused = 2, kCoarse = 3, kPausing = 4;
 
 // the plan on the device
 struct HierGraph {
@@ -50,7 +51,8 @@ struct HierArgs {
   int absent_words;
   unsigned long long* w;                      // [slot][3 arcs] integer weights: down, up, closed
   unsigned long long* mid;      // [slot][3 arcs] the two slots a shortcut splits into
-  unsigned long long* flow;     // [slot][3 arcs] fixed-point volumes (all zero between iterations)
+  unsigned long long* flow;     // [slot][3 arcs] fixed-point volumes (all zero between loadings,
+                                // so scenarios can take turns in a slot)
   unsigned long long* d0;                     // [slot][origin][climb] labels of the climb
   int* from;                    // [slot][origin][climb] the up arc each of them came over
   unsigned char* via;           // [slot][origin][climb] later row of the chunk it came from, or 0xff

@@ -347,15 +347,7 @@ bool Ctx::hier_pays(int nscen, int levels, double relaxations, int arcs) const {
 // The path kernels of the next iterations of nscen scenarios, and their buffers.
 int Ctx::choose_paths(int nscen) {
   bool on = hier && hier_pays(nscen);
-  if (on && hier_cap < nscen) {
-    if (gexec) cudaGraphExecDestroy(gexec);
-    gexec = nullptr;
-    if (ensure_hier(nscen) != TAPGPU_OK) {  // no room: the label-correction kernels
-      cudaGetLastError();
-      release_hier();
-      on = false;
-    }
-  }
+  if (on) on = have_hier(nscen);  // (no room: the label-correction kernels)
   if (!on) {
     const int rc = ensure_legacy(S_cap);
     if (rc != TAPGPU_OK) {  // (the next call starts from its own number of scenarios)
@@ -369,6 +361,17 @@ int Ctx::choose_paths(int nscen) {
   }
   hier_on = on;
   return TAPGPU_OK;
+}
+
+// Whether the hierarchy's buffers for nscen scenarios are there, or could be made.
+bool Ctx::have_hier(int nscen) {
+  if (hier_cap >= nscen) return true;
+  if (gexec) cudaGraphExecDestroy(gexec);
+  gexec = nullptr;
+  if (ensure_hier(nscen) == TAPGPU_OK) return true;
+  cudaGetLastError();
+  release_hier();
+  return false;
 }
 
 // The weight records and the label buffer of the label-correction kernels.
@@ -652,9 +655,9 @@ int Ctx::ensure_hier(int S) {
   const size_t climb = static_cast<size_t>(Z) * hg.climb;
   // labels of the top rows for every origin (padded to whole groups)
   const size_t top = static_cast<size_t>(h_width) * hg.top_rows;
-  // at most 24 GiB of per-scenario buffers; more scenarios take turns in them
+  // per-scenario buffers within hier_bytes; more scenarios take turns in them
   const size_t per = arcs3 * 32 + climb * 21 + top * 18;
-  hier_slots = static_cast<int>(std::max<size_t>(1, std::min<size_t>(S, (size_t(24) << 30) / per)));
+  hier_slots = static_cast<int>(std::max<size_t>(1, std::min<size_t>(S, hier_bytes / per)));
   const size_t ns = static_cast<size_t>(hier_slots), nc = ns * top;
   TG_TRY(alloc_n(&h_w, ns * arcs3));
   TG_TRY(alloc_n(&h_mid, ns * arcs3));
@@ -771,8 +774,6 @@ int Ctx::hier_load_api(bool* loaded) {
     if (st.done == kPaused) st.u_exp -= kHierRetryBits;
     st.done = 0;
     st.maxlab = 0;
-    TG_CUDA(cudaMemsetAsync(h_flow, 0, static_cast<size_t>(hier_slots) * 3 * hg.arcs *
-                                           sizeof(unsigned long long), stream));
   }
   return TAPGPU_OK;
 }
@@ -801,10 +802,6 @@ int Ctx::resume_paused(int S, std::vector<ScenState>& st) {
     TG_CUDA(cudaMemcpyAsync(state + s, &st[s], sizeof(ScenState), cudaMemcpyHostToDevice, stream));
   }
   if (!any) return TAPGPU_OK;
-  // a paused scenario's volumes stayed where they were
-  TG_CUDA(cudaMemsetAsync(h_flow, 0,
-                          static_cast<size_t>(hier_slots) * 3 * hg.arcs * sizeof(unsigned long long),
-                          stream));
   TG_CUDA(cudaStreamSynchronize(stream));
   if (legacy.empty()) return TAPGPU_OK;
   TG_TRY(ensure_legacy(S_cap));
@@ -1004,8 +1001,6 @@ int Ctx::begin_paths(int nscen) {
                                 stream));
       }
       if (!paused) return TAPGPU_OK;
-      TG_CUDA(cudaMemsetAsync(h_flow, 0, static_cast<size_t>(hier_slots) * 3 * hg.arcs *
-                                             sizeof(unsigned long long), stream));
       TG_CUDA(cudaStreamSynchronize(stream));
     }
     TG_TRY(ensure_legacy(S_cap));  // (which also reports a missing path)
@@ -2205,7 +2200,7 @@ int tapgpu_aon(tapgpu_ctx* ctx, const double* weights, double* volume) {
   TG_CUDA(cudaMemsetAsync(c->api_yfx, 0, sizeof(unsigned long long) * c->M, c->stream));
   TG_CUDA(cudaMemsetAsync(c->err, 0, sizeof(int), c->stream));
   bool loaded = false;
-  if (c->hier && c->hier_cap >= 1 && c->hier_pays(1)) {
+  if (c->hier && c->hier_pays(1) && c->have_hier(1)) {
     TG_TRY(c->hier_load_api(&loaded));
     if (!loaded)
       TG_CUDA(cudaMemsetAsync(c->api_yfx, 0, sizeof(unsigned long long) * c->M, c->stream));
@@ -2270,6 +2265,20 @@ int tapgpu_run_iterations(tapgpu_ctx* ctx, int iters) {
     TG_TRY(c->set_active(active));
     TG_TRY(c->run_graph(std::max(1, std::min(per, left)), static_cast<int>(active.size())));
   }
+}
+
+int tapgpu_set_hierarchy_limit(tapgpu_ctx* ctx, int64_t bytes) {
+  if (!ctx) return TAPGPU_ERR_ARG;
+  Ctx* c = ctx->c;
+  TG_CUDA(cudaSetDevice(c->device));
+  TG_CUDA(cudaStreamSynchronize(c->stream));
+  c->hier_bytes = bytes > 0 ? static_cast<size_t>(bytes) : tapgpu::kHierBytes;
+  if (c->gexec) {  // captured launches hold the buffers' addresses
+    cudaGraphExecDestroy(c->gexec);
+    c->gexec = nullptr;
+  }
+  c->release_hier();
+  return TAPGPU_OK;
 }
 
 int tapgpu_set_timing(tapgpu_ctx* ctx, int on) {

@@ -20,6 +20,9 @@ struct DevMem {
   size_t bytes = 0;
 };
 
+// default bound of the elimination hierarchy's per-scenario buffers
+constexpr size_t kHierBytes = size_t(24) << 30;
+
 struct Ctx {
   // sizes (internal link order: sorted by (init, term))
   int N = 0, n1 = 0, M = 0, Z = 0, F = 0;
@@ -151,7 +154,8 @@ struct Ctx {
   int* h_od_dest = nullptr;      // destination index of each OD entry or -1
   int h_dests = 0, h_width = 0;  // demand by destination: [h_dests][h_width]
   unsigned long long *h_dem = nullptr, *h_sc_dem = nullptr;
-  int hier_slots = 0;            // scenarios the buffers below hold
+  size_t hier_bytes = kHierBytes;  // bound of the buffers below
+  int hier_slots = 0;            // scenarios they hold
   unsigned long long *h_w = nullptr, *h_d0 = nullptr, *h_fup = nullptr;
   unsigned long long *h_dlab = nullptr, *h_vol = nullptr;
   unsigned long long *h_mid = nullptr, *h_flow = nullptr;
@@ -254,6 +258,7 @@ struct Ctx {
   int hier_demand(const long long* dev_q, int nscen, unsigned long long** dem);
   void release_hier();
   int ensure_hier(int S);
+  bool have_hier(int nscen);
   bool hier_pays(int nscen, int levels, double relaxations, int arcs) const;
   bool hier_pays(int nscen) const {
     return hier_pays(nscen, static_cast<int>(h_tile_ptr.size()) - 1, hier_relaxations, hg.arcs);
@@ -264,7 +269,9 @@ struct Ctx {
   void release_records();
   int ensure_labels();
   // the arrays of the last solve are there
-  bool can_iterate() const { return S_cap > 0 && (hier_on || records_ready); }
+  bool can_iterate() const {
+    return S_cap > 0 && (hier_on ? hier_cap > 0 : records_ready);
+  }
   int enqueue_hier(int nscen, const double* cost, long long stride, cudaEvent_t between = nullptr);
   HierArgs hier_args(const double* cost, long long stride) const;
   int hier_load_api(bool* loaded);

@@ -279,6 +279,11 @@ class Solver:
     def run_iterations(self, iters: int):
         K.check(self.L.tapgpu_run_iterations(self.h, int(iters)))
 
+    def set_hierarchy_limit(self, nbytes: int = 0):
+        """Bound of the elimination hierarchy's per-scenario buffers (0: 24 GiB); more
+        scenarios than fit take turns in them."""
+        K.check(self.L.tapgpu_set_hierarchy_limit(self.h, int(nbytes)))
+
     def set_timing(self, on: bool = True):
         K.check(self.L.tapgpu_set_timing(self.h, 1 if on else 0))
 
