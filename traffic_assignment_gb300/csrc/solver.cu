@@ -2348,34 +2348,32 @@ int tapgpu_profile_iteration(tapgpu_ctx* ctx, int reps, float* ms) {
   for (auto& e : ev) TG_CUDA(cudaEventCreate(&e));
   double acc[5] = {0, 0, 0, 0, 0};
   int rc = TAPGPU_OK;
-  for (int r = 0; r < reps && rc == TAPGPU_OK; ++r) {
+  const int64_t tasks = c->Z;
+  if (!c->hier_on && tasks > c->dist_tasks) rc = TAPGPU_ERR_UNSUPPORTED;
+  int pauses = 0;
+  for (int r = 0; r < reps && rc == TAPGPU_OK;) {
     cudaEventRecord(ev[0], c->stream);
-    const int64_t tasks = c->Z;
     if (c->hier_on) {
       rc = c->enqueue_hier(1, c->t, c->M, ev[1]);
       if (rc != TAPGPU_OK) break;
       cudaEventRecord(ev[2], c->stream);
     } else {
-    tapgpu::PathArgs a = c->path_args(1);
-    a.task_end = static_cast<int>(tasks);
-    cudaMemsetAsync(c->counters, 0, 2 * sizeof(int), c->stream);
-    a.counter = c->counters;
-    a.scratch_stride = static_cast<long long>(tapgpu::sssp_smem_bytes(c->n1, c->fp64, c->sssp_variant, c->M));
-    a.e32 = c->fp64 ? nullptr : c->e32;
-    a.r32 = c->fp64 ? nullptr : c->r32;
-    a.w64 = c->fp64 ? c->w64 : nullptr;
-    if (tasks > c->dist_tasks) {
-      rc = TAPGPU_ERR_UNSUPPORTED;
-      break;
-    }
-    tapgpu::launch_sssp(a, c->fp64, std::min<int64_t>(c->sssp_grid, tasks), c->sssp_block,
-                        c->sssp_smem, c->sssp_variant, c->stream);
-    cudaEventRecord(ev[1], c->stream);
-    a.counter = c->counters + 1;
-    a.scratch_stride = static_cast<long long>(tapgpu::aon_smem_bytes(c->n1, c->fp64, c->aon_c64));
-    tapgpu::launch_aon(a, c->fp64, std::min<int64_t>(c->aon_grid, tasks), c->aon_block,
-                       c->aon_smem, c->stream);
-    cudaEventRecord(ev[2], c->stream);
+      tapgpu::PathArgs a = c->path_args(1);
+      a.task_end = static_cast<int>(tasks);
+      cudaMemsetAsync(c->counters, 0, 2 * sizeof(int), c->stream);
+      a.counter = c->counters;
+      a.scratch_stride = static_cast<long long>(tapgpu::sssp_smem_bytes(c->n1, c->fp64, c->sssp_variant, c->M));
+      a.e32 = c->fp64 ? nullptr : c->e32;
+      a.r32 = c->fp64 ? nullptr : c->r32;
+      a.w64 = c->fp64 ? c->w64 : nullptr;
+      tapgpu::launch_sssp(a, c->fp64, std::min<int64_t>(c->sssp_grid, tasks), c->sssp_block,
+                          c->sssp_smem, c->sssp_variant, c->stream);
+      cudaEventRecord(ev[1], c->stream);
+      a.counter = c->counters + 1;
+      a.scratch_stride = static_cast<long long>(tapgpu::aon_smem_bytes(c->n1, c->fp64, c->aon_c64));
+      tapgpu::launch_aon(a, c->fp64, std::min<int64_t>(c->aon_grid, tasks), c->aon_block,
+                         c->aon_smem, c->stream);
+      cudaEventRecord(ev[2], c->stream);
     }
     tapgpu::LinkArgs la = c->link_args(1);
     for (la.pass = 0; la.pass < c->grid_passes(); ++la.pass)
@@ -2388,6 +2386,14 @@ int tapgpu_profile_iteration(tapgpu_ctx* ctx, int reps, float* ms) {
       rc = TAPGPU_ERR_CUDA;
       break;
     }
+    if (c->hier_on) {  // an iteration that paused is repeated, not counted
+      rc = c->read_states(1, st);
+      if (rc != TAPGPU_OK) break;
+      if (st[0].done > 1) {
+        rc = ++pauses <= reps + 64 ? c->resume_paused(1, st) : TAPGPU_ERR_NO_CONVERGENCE;
+        continue;
+      }
+    }
     float t;
     for (int i = 0; i < 4; ++i) {
       cudaEventElapsedTime(&t, ev[i], ev[i + 1]);
@@ -2395,6 +2401,7 @@ int tapgpu_profile_iteration(tapgpu_ctx* ctx, int reps, float* ms) {
     }
     cudaEventElapsedTime(&t, ev[0], ev[4]);
     acc[4] += t;
+    ++r;
   }
   for (auto& e : ev) cudaEventDestroy(e);
   if (rc != TAPGPU_OK) return rc;
