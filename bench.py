@@ -91,7 +91,7 @@ class Dist:
 
 
 # bytes of one scenario's device state record (sizeof the struct)
-SCEN_STATE_BYTES = 152
+SCEN_STATE_BYTES = 160
 
 
 def shard_scenarios(net, count, rank):

@@ -57,6 +57,7 @@ struct ScenState {
   int max_iters;   // <= 0: no cap
   int u_exp;       // integer path labels: costs are scaled by 2^u_exp
   unsigned long long maxlab;  // largest integer label of the iteration
+  unsigned long long minlab;  // and its smallest one above zero, all ones: none
   double target_relgap;
   double relgap, best_lb, obj, gap, lambda, vht, avg_excess, g0;
   double vht_end;  // VHT at the current x with the current costs

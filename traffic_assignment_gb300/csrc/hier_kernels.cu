@@ -64,6 +64,11 @@ using Int = unsigned long long;  // labels, weights and volumes
 constexpr Int kInf = 1ull << 62;
 constexpr int kBits = 55;     // the largest label has kBits + 1 bits next time
 constexpr int kMinBits = 53;  // with fewer the iteration is repeated
+// The smallest label of a pair with demand has at least kLeastBits + 1 bits, so
+// a link's rounding is at most 2^-41 of any path's cost; else the label-correction
+// kernels take the iteration (kSpread).  City networks, cold and warm, have pairs
+// from 1 to 2^7 .. 2^10: their smallest labels keep 46 to 49 bits.
+constexpr int kLeastBits = 40;
 
 __device__ __forceinline__ Int addmin(Int a, Int b, Int c) {
   const Int s = a + b;
@@ -89,14 +94,17 @@ __device__ __forceinline__ void weights4(const Int* p, Int (&w)[4]) {
   w[3] = y.y;
 }
 
-// integer weight of link k of a scenario; kInf when absent or out of range
+// integer weight of link k of a scenario; kInf when absent or out of range, zero
+// for a zero cost only (a label of zero is exact)
 __device__ __forceinline__ Int link_weight(const HierArgs& a, int scen, int k, double scale) {
   if (a.absent &&
       ((__ldg(a.absent + static_cast<size_t>(scen) * a.absent_words + (k >> 5)) >> (k & 31)) & 1u))
     return kInf;
-  const double v =
-      __dmul_rn(a.cost[static_cast<size_t>(scen) * static_cast<size_t>(a.cost_stride) + k], scale);
-  return v < static_cast<double>(kInf) ? __double2ull_rn(v) : kInf;
+  const double c = a.cost[static_cast<size_t>(scen) * static_cast<size_t>(a.cost_stride) + k];
+  const double v = __dmul_rn(c, scale);
+  if (!(v < static_cast<double>(kInf))) return kInf;
+  const Int w = __double2ull_rn(v);
+  return w == 0 && c > 0.0 ? Int(1) : w;
 }
 
 // the two arc slots (planes included) an arc splits into
@@ -849,7 +857,7 @@ __device__ __forceinline__ Lane lane_of(const HierArgs& a, int slot, int grp) {
 
 // a lane's demand at a destination: sums up what it saw of the labels
 struct DemandAt {
-  Int largest = 0;
+  Int largest = 0, least = ~Int(0);
   bool out_of_range = false;
   // demand q at label x (all ones: some, below the unit)
   __device__ __forceinline__ Int take(Int q, Int x) {
@@ -859,6 +867,7 @@ struct DemandAt {
       return 0;
     }
     if (x > largest) largest = x;
+    if (x - 1 < least) least = x - 1;  // (zero wraps round)
     return q == ~Int(0) ? Int(0) : q;
   }
   // by whole warps
@@ -871,6 +880,13 @@ struct DemandAt {
       if (n > x) x = n;
     }
     if ((threadIdx.x & 31) == 0 && x) atomicMax(&st.maxlab, x);
+    x = least;
+#pragma unroll
+    for (int z = 16; z >= 1; z >>= 1) {
+      const Int n = __shfl_xor_sync(kFull, x, z);
+      if (n < x) x = n;
+    }
+    if ((threadIdx.x & 31) == 0 && x != ~Int(0)) atomicMin(&st.minlab, x + 1);
   }
 };
 
@@ -1521,9 +1537,14 @@ __global__ void __launch_bounds__(kElimBlock) k_hier_exponents(HierArgs a) {
   if (st.done || !st.maxlab) return;
   const int top = 63 - __clzll(static_cast<long long>(st.maxlab));
   const int u_exp = max(-kMaxExp, min(kMaxExp, st.u_exp + kBits - top));
-  if (top < kMinBits && u_exp != st.u_exp) st.done = kCoarse;
+  const bool spread = st.minlab < (Int(1) << kLeastBits);
+  if ((top < kMinBits || (spread && top < kBits)) && u_exp != st.u_exp)
+    st.done = kCoarse;
+  else if (spread)
+    st.done = kSpread;
   st.u_exp = u_exp;
   st.maxlab = 0ull;
+  st.minlab = ~Int(0);
 }
 
 template <typename Fn>

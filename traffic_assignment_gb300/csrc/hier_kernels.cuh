@@ -8,8 +8,9 @@ namespace tapgpu {
 
 // ScenState::done: labels left the integer range, or used too little of it
 // (see hier_kernels.cu); kPausing: left it in the iteration under way, whose
-// loading empties the scenario's buffers and then makes it kPaused
-constexpr int kPaused = 2, kCoarse = 3, kPausing = 4;
+// loading empties the scenario's buffers and then makes it kPaused; kSpread: the
+// labels of some pairs have too few bits beside the largest one
+constexpr int kPaused = 2, kCoarse = 3, kPausing = 4, kSpread = 5;
 
 // the plan on the device
 struct HierGraph {

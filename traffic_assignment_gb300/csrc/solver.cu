@@ -742,6 +742,18 @@ HierArgs Ctx::hier_args(const double* cost, long long stride) const {
 constexpr int kHierRetries = 4;
 constexpr int kHierRetryBits = 5;
 
+// A paused scenario's state for its next try; false where the label-correction
+// kernels take over.
+static bool next_try(ScenState& st, int tries) {
+  const int why = st.done;
+  st.done = 0;
+  st.maxlab = 0;
+  st.minlab = ~0ull;
+  if (why == kSpread || tries >= kHierRetries) return false;
+  if (why == kPaused) st.u_exp -= kHierRetryBits;  // (of a coarse one the device set it)
+  return true;
+}
+
 // One loading of the base demand at the costs of an API call (api_w64) into
 // api_yfx, with a state of its own.  *loaded stays false where the labels do
 // not fit after kHierRetries exponents: the label-correction kernels' case.
@@ -758,7 +770,8 @@ int Ctx::hier_load_api(bool* loaded) {
   ScenState st;
   std::memset(&st, 0, sizeof(st));
   st.u_exp = u_exp0;
-  for (int tries = 0; tries <= kHierRetries; ++tries) {
+  st.minlab = ~0ull;
+  for (int tries = 0;; ++tries) {
     TG_CUDA(cudaMemcpyAsync(api_state, &st, sizeof(st), cudaMemcpyHostToDevice, stream));
     const int levels = static_cast<int>(h_tile_ptr.size()) - 1;
     TG_CUDA(launch_hier_eliminate(a, levels, h_tile_ptr.data(), stream));
@@ -771,49 +784,66 @@ int Ctx::hier_load_api(bool* loaded) {
       *loaded = true;
       return TAPGPU_OK;
     }
-    if (st.done == kPaused) st.u_exp -= kHierRetryBits;
-    st.done = 0;
-    st.maxlab = 0;
+    if (!next_try(st, tries)) return TAPGPU_OK;
   }
-  return TAPGPU_OK;
 }
 
 // Scenarios that left the integers' range repeat their iteration at a smaller
 // exponent (those that used too little of it have their new one); one that
-// does so repeatedly takes this iteration with the label-correction kernels,
-// which also report a missing path.
+// does so repeatedly, or whose labels are spread too far, takes this iteration
+// with the label-correction kernels, which also report a missing path.
 int Ctx::resume_paused(int S, std::vector<ScenState>& st) {
   if (!hier_on) return TAPGPU_OK;
-  std::vector<int> legacy;
+  std::vector<int> corrected;
   bool any = false;
-  hier_retry.resize(S, {-1, 0});
+  hier_course.resize(S);
   for (int s = 0; s < S; ++s) {
     if (st[s].done <= 1) continue;
     any = true;
-    const bool coarse = st[s].done == kCoarse;  // (its exponent is set)
-    auto& r = hier_retry[s];
-    if (r.first != st[s].iter) r = {st[s].iter, 0};
-    st[s].done = 0;
-    st[s].maxlab = 0;
-    if (++r.second > kHierRetries)
-      legacy.push_back(s);
-    else if (!coarse)
-      st[s].u_exp -= kHierRetryBits;
+    auto& c = hier_course[s];
+    if (c.iter != st[s].iter) {
+      c.iter = st[s].iter;
+      c.pauses = 0;
+    }
+    if (st[s].done == kSpread) ++c.spread;
+    if (!next_try(st[s], c.pauses++)) corrected.push_back(s);
     TG_CUDA(cudaMemcpyAsync(state + s, &st[s], sizeof(ScenState), cudaMemcpyHostToDevice, stream));
   }
   if (!any) return TAPGPU_OK;
   TG_CUDA(cudaStreamSynchronize(stream));
-  if (legacy.empty()) return TAPGPU_OK;
-  TG_TRY(ensure_legacy(S_cap));
-  TG_TRY(set_active(legacy));
-  const int n = static_cast<int>(legacy.size());
-  LinkArgs la = link_args(n, true);
-  TG_CUDA(cudaMemsetAsync(yfx, 0, sizeof(unsigned long long) * static_cast<size_t>(S_cap) * M, stream));
-  TG_CUDA(launch_records(la, link_grid, stream));
-  TG_TRY(enqueue_paths(n, true, e32, r32, w64, yfx, true));
-  TG_TRY(enqueue_tail(n));
+  if (corrected.empty()) return TAPGPU_OK;
+  TG_TRY(run_corrected(corrected, 1));
   TG_TRY(sync_check());
   return read_states(S, st);
+}
+
+// Iterations of the listed scenarios with the label-correction kernels while
+// the others are on the hierarchy.
+int Ctx::run_corrected(const std::vector<int>& list, int iters) {
+  TG_TRY(ensure_legacy(S_cap));
+  TG_TRY(set_active(list));
+  const int n = static_cast<int>(list.size());
+  // (the hierarchy's loading writes volumes, that of these kernels adds to them)
+  TG_CUDA(cudaMemsetAsync(yfx, 0, sizeof(unsigned long long) * static_cast<size_t>(S_cap) * M, stream));
+  TG_CUDA(launch_records(link_args(n, true), link_grid, stream));
+  for (int i = 0; i < iters; ++i) {
+    TG_TRY(enqueue_paths(n, true, e32, r32, w64, yfx, true));
+    TG_TRY(enqueue_tail(n, true));
+  }
+  return TAPGPU_OK;
+}
+
+// Iterations of the active scenarios.  One whose labels were spread too far in
+// kSpreadIters iterations keeps the label-correction kernels for the rest of
+// the solve: trying the hierarchy first costs an iteration more every time.
+int Ctx::run_active(const std::vector<int>& active, int iters) {
+  std::vector<int> swept, corrected;
+  for (int s : active) (on_hierarchy(s) || !hier_on ? swept : corrected).push_back(s);
+  if (!swept.empty()) {
+    TG_TRY(set_active(swept));
+    TG_TRY(run_graph(iters, static_cast<int>(swept.size())));
+  }
+  return corrected.empty() ? TAPGPU_OK : run_corrected(corrected, iters);
 }
 
 int Ctx::set_active(const std::vector<int>& active) {
@@ -950,8 +980,8 @@ int Ctx::enqueue_iteration(int nscen) {
 }
 
 // line search and step of an iteration
-int Ctx::enqueue_tail(int nscen) {
-  LinkArgs la = link_args(nscen);
+int Ctx::enqueue_tail(int nscen, bool records) {
+  LinkArgs la = link_args(nscen, records);
   if (M <= kSmallTail) {  // small networks: the line search and the step in one launch
     TG_TRY(mark(2, true));
     TG_CUDA(launch_fw_tail_small(la, stream));
@@ -982,32 +1012,36 @@ int Ctx::enqueue_initial(int nscen, bool warm) {
   return TAPGPU_OK;
 }
 
-// All-or-nothing at free-flow costs of the first nscen entries of scen_list
+// All-or-nothing at free-flow costs of scenarios 0 .. nscen-1
 int Ctx::begin_paths(int nscen) {
-  if (hier_on) {
-    const LinkParams lp = link_params();
-    std::vector<ScenState> st;
-    for (int tries = 0; tries <= kHierRetries; ++tries) {
-      TG_TRY(enqueue_hier(nscen, lp.fft, lp.stride));
-      TG_TRY(read_states(nscen, st));
-      bool paused = false;
-      for (int s = 0; s < nscen; ++s) {
-        if (st[s].done <= 1) continue;
-        paused = true;
-        if (st[s].done == kPaused) st[s].u_exp -= kHierRetryBits;
-        st[s].done = 0;
-        st[s].maxlab = 0;
-        TG_CUDA(cudaMemcpyAsync(state + s, &st[s], sizeof(ScenState), cudaMemcpyHostToDevice,
-                                stream));
-      }
-      if (!paused) return TAPGPU_OK;
-      TG_CUDA(cudaStreamSynchronize(stream));
+  std::vector<int> all(nscen);
+  std::iota(all.begin(), all.end(), 0);
+  std::vector<int> corrected;
+  if (!hier_on) corrected = all;
+  const LinkParams lp = link_params();
+  std::vector<ScenState> st;
+  std::vector<int> todo = hier_on ? all : std::vector<int>(), again;
+  for (int tries = 0; !todo.empty(); ++tries, todo.swap(again)) {
+    TG_TRY(set_active(todo));
+    TG_TRY(enqueue_hier(static_cast<int>(todo.size()), lp.fft, lp.stride));
+    TG_TRY(read_states(nscen, st));
+    again.clear();
+    for (int s : todo) {
+      if (st[s].done <= 1) continue;
+      (next_try(st[s], tries) ? again : corrected).push_back(s);
+      TG_CUDA(cudaMemcpyAsync(state + s, &st[s], sizeof(ScenState), cudaMemcpyHostToDevice, stream));
     }
-    TG_TRY(ensure_legacy(S_cap));  // (which also reports a missing path)
+    TG_CUDA(cudaStreamSynchronize(stream));
   }
-  TG_CUDA(launch_set_costs(link_args(nscen, true), link_grid, stream));
-  count_launches(1);
-  return enqueue_paths(nscen, true, e32, r32, w64, yfx, true);
+  if (!corrected.empty()) {  // (these kernels also report a missing path)
+    const int n = static_cast<int>(corrected.size());
+    TG_TRY(ensure_legacy(S_cap));
+    TG_TRY(set_active(corrected));
+    TG_CUDA(launch_set_costs(link_args(n, true), link_grid, stream));
+    count_launches(1);
+    TG_TRY(enqueue_paths(n, true, e32, r32, w64, yfx, true));
+  }
+  return set_active(all);
 }
 
 int Ctx::run_graph(int iters, int nscen) {
@@ -1393,8 +1427,9 @@ static int upload_states(Ctx* c, int S, int max_iters, double target) {
     s.relgap = DBL_MAX;
     s.best_lb = -DBL_MAX;
     s.u_exp = c->u_exp0;
+    s.minlab = ~0ull;
   }
-  c->hier_retry.clear();
+  c->hier_course.clear();
   TG_CUDA(cudaMemcpyAsync(c->state, st.data(), sizeof(ScenState) * S, cudaMemcpyHostToDevice,
                           c->stream));
   TG_CUDA(cudaMemsetAsync(c->err, 0, sizeof(int), c->stream));
@@ -1432,8 +1467,7 @@ static int iterate_until_done(Ctx* c, int S, int max_iters, std::vector<ScenStat
     for (int s = 0; s < S; ++s)
       if (!st[s].done) active.push_back(s);
     if (active.empty()) break;
-    TG_TRY(c->set_active(active));
-    TG_TRY(c->run_graph(per, static_cast<int>(active.size())));
+    TG_TRY(c->run_active(active, per));
   }
   return TAPGPU_OK;
 }
@@ -1558,8 +1592,7 @@ int tapgpu_solve_advance(tapgpu_ctx* ctx, int max_new_iters, int* done, tapgpu_r
   if (c->solve_max_iters > 0) n = std::max(1, std::min(n, c->solve_max_iters - st[0].iter));
   const int goal = st[0].iter + n;
   while (!st[0].done && st[0].iter < goal) {  // (again after a pause)
-    TG_TRY(c->set_active({0}));
-    TG_TRY(c->run_graph(goal - st[0].iter, 1));
+    TG_TRY(c->run_active({0}, goal - st[0].iter));
     TG_TRY(c->read_states(1, st));
     TG_TRY(c->sync_check());
     TG_TRY(c->resume_paused(1, st));
@@ -1800,6 +1833,7 @@ int tapgpu_solve_scenarios(tapgpu_ctx* ctx, int num_scen, const int64_t* scen_pt
     // free-flow all-or-nothing does not depend on capacity: load scenario 0
     // once and start every scenario from it
     TG_TRY(c->begin_paths(1));
+    TG_TRY(c->set_active(all));
     if (c->hier_on && num_scen > 1) {  // its exponent too
       std::vector<tapgpu::ScenState> st0;
       TG_TRY(c->read_states(num_scen, st0));
@@ -2244,9 +2278,8 @@ int tapgpu_run_iterations(tapgpu_ctx* ctx, int iters) {
                           cudaMemcpyHostToDevice, c->stream));
   std::vector<int> all(S);
   std::iota(all.begin(), all.end(), 0);
-  TG_TRY(c->set_active(all));
   const int per = tapgpu::equal_parts(iters, c->opt.iters_per_launch > 0 ? c->opt.iters_per_launch : 8);
-  for (int done = 0; done < iters; done += per) TG_TRY(c->run_graph(per, S));
+  for (int done = 0; done < iters; done += per) TG_TRY(c->run_active(all, per));
   if (!c->hier_on) return TAPGPU_OK;
   for (;;) {  // scenarios that paused on the way take their remaining iterations
     TG_TRY(c->read_states(S, st));
@@ -2262,8 +2295,7 @@ int tapgpu_run_iterations(tapgpu_ctx* ctx, int iters) {
         left = std::max(left, st[s].max_iters - st[s].iter);
       }
     if (active.empty()) return TAPGPU_OK;
-    TG_TRY(c->set_active(active));
-    TG_TRY(c->run_graph(std::max(1, std::min(per, left)), static_cast<int>(active.size())));
+    TG_TRY(c->run_active(active, std::max(1, std::min(per, left))));
   }
 }
 
@@ -2349,11 +2381,16 @@ int tapgpu_profile_iteration(tapgpu_ctx* ctx, int reps, float* ms) {
   double acc[5] = {0, 0, 0, 0, 0};
   int rc = TAPGPU_OK;
   const int64_t tasks = c->Z;
-  if (!c->hier_on && tasks > c->dist_tasks) rc = TAPGPU_ERR_UNSUPPORTED;
   int pauses = 0;
   for (int r = 0; r < reps && rc == TAPGPU_OK;) {
+    const bool swept = c->on_hierarchy(0);
+    if (!swept && tasks > c->dist_tasks) {
+      rc = TAPGPU_ERR_UNSUPPORTED;
+      break;
+    }
+    if (!swept && c->hier_on) tapgpu::launch_records(c->link_args(1, true), c->link_grid, c->stream);
     cudaEventRecord(ev[0], c->stream);
-    if (c->hier_on) {
+    if (swept) {
       rc = c->enqueue_hier(1, c->t, c->M, ev[1]);
       if (rc != TAPGPU_OK) break;
       cudaEventRecord(ev[2], c->stream);
@@ -2386,12 +2423,12 @@ int tapgpu_profile_iteration(tapgpu_ctx* ctx, int reps, float* ms) {
       rc = TAPGPU_ERR_CUDA;
       break;
     }
-    if (c->hier_on) {  // an iteration that paused is repeated, not counted
+    if (swept) {  // an iteration that paused is repeated, not counted
       rc = c->read_states(1, st);
       if (rc != TAPGPU_OK) break;
       if (st[0].done > 1) {
         rc = ++pauses <= reps + 64 ? c->resume_paused(1, st) : TAPGPU_ERR_NO_CONVERGENCE;
-        continue;
+        continue;  // (the list of active scenarios stays {0})
       }
     }
     float t;

@@ -22,6 +22,8 @@ struct DevMem {
 
 // default bound of the elimination hierarchy's per-scenario buffers
 constexpr size_t kHierBytes = size_t(24) << 30;
+// iterations of a scenario after which its spread labels keep it off the hierarchy
+constexpr int kSpreadIters = 2;
 
 struct Ctx {
   // sizes (internal link order: sorted by (init, term))
@@ -162,7 +164,15 @@ struct Ctx {
   unsigned char* h_via = nullptr;
   int *h_from = nullptr, *h_list = nullptr, *h_list_n = nullptr;
   unsigned short* h_arr = nullptr;
-  std::vector<std::pair<int, int>> hier_retry;  // per scenario: iteration, pauses in it
+  struct HierCourse {
+    int iter = -1, pauses = 0;   // the iteration that paused last, and how often
+    int spread = 0;              // iterations given to the label-correction kernels for their spread
+  };
+  std::vector<HierCourse> hier_course;  // by scenario, of the present solve
+  // whether scenario s takes its iterations on the hierarchy
+  bool on_hierarchy(int s) const {
+    return hier_on && (s >= static_cast<int>(hier_course.size()) || hier_course[s].spread < kSpreadIters);
+  }
 
   cudaStream_t stream = nullptr;
   cudaGraphExec_t gexec = nullptr;
@@ -251,7 +261,7 @@ struct Ctx {
                     unsigned long long* ydst, bool use_state);
   int enqueue_iteration(int nscen);
   int enqueue_initial(int nscen, bool warm);
-  int enqueue_tail(int nscen);
+  int enqueue_tail(int nscen, bool records = false);
   int run_graph(int iters, int nscen);
   int hier_plan(const HierPlan* plan, const std::vector<int>& odest, const std::vector<int>& optr,
                 const std::vector<double>& odem);
@@ -278,6 +288,8 @@ struct Ctx {
   int begin_paths(int nscen);
   int set_active(const std::vector<int>& active);
   int resume_paused(int S, std::vector<ScenState>& st);
+  int run_corrected(const std::vector<int>& list, int iters);
+  int run_active(const std::vector<int>& active, int iters);
   int sync_check();
   int read_states(int S, std::vector<ScenState>& out);
 };
