@@ -2115,7 +2115,7 @@ int tapgpu_sssp(tapgpu_ctx* ctx, const double* weights, const int64_t* srcs, int
     c->api_src = c->pred_buf = nullptr;
     c->api_pred = nullptr;
     c->api_rows = 0;
-    c->api_pred_rows = std::max<int64_t>(1, std::min<int64_t>(rows, (int64_t(64) << 20) / (8 * n1)));
+    c->api_pred_rows = tapgpu::rows_at_once(rows, n1);
     TG_TRY(c->alloc_n(&c->api_src, static_cast<size_t>(rows)));
     TG_TRY(c->alloc_n(&c->pred_buf, static_cast<size_t>(rows) * n1));
     TG_TRY(c->alloc_n(&c->api_pred, static_cast<size_t>(c->api_pred_rows) * n1));

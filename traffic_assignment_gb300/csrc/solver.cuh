@@ -1,5 +1,6 @@
 // solver.cuh - host-side solver context behind the tapgpu_* C ABI.
 #pragma once
+#include <algorithm>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -24,6 +25,12 @@ struct DevMem {
 constexpr size_t kHierBytes = size_t(24) << 30;
 // iterations of a scenario after which its spread labels keep it off the hierarchy
 constexpr int kSpreadIters = 2;
+
+// predecessor rows of n1 64-bit link indices that the shortest-path API widens at
+// once: 64 MiB of them, one at least (n1 up to 2^30 + 1)
+inline int64_t rows_at_once(int64_t rows, int n1) {
+  return std::max<int64_t>(1, std::min<int64_t>(rows, (int64_t(64) << 20) / (int64_t(8) * n1)));
+}
 
 struct Ctx {
   // sizes (internal link order: sorted by (init, term))
