@@ -397,6 +397,9 @@ int tapgpu_get_path_stats(tapgpu_ctx *ctx, int64_t *out);
 /* Bound in bytes of the elimination hierarchy's per-scenario buffers (FP64
  * iterations; default 24 GiB, which bytes <= 0 restores): of a batch that needs
  * more, scenarios take turns in what the bound holds, at least one at a time.
+ * Beside them a table of the demand by destination and origin is held, 8 bytes
+ * for every pair of zones and demand scenario; batches whose table exceeds 24
+ * GiB, and those that find no memory, are iterated by label correction.
  * Gives the present buffers back; the next solve makes its own. */
 int tapgpu_set_hierarchy_limit(tapgpu_ctx *ctx, int64_t bytes);
 

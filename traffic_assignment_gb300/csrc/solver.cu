@@ -346,8 +346,8 @@ bool Ctx::hier_pays(int nscen, int levels, double relaxations, int arcs) const {
 
 // The path kernels of the next iterations of nscen scenarios, and their buffers.
 int Ctx::choose_paths(int nscen) {
-  bool on = hier && hier_pays(nscen);
-  if (on) on = have_hier(nscen);  // (no room: the label-correction kernels)
+  bool on = false;  // (no room: the label-correction kernels)
+  if (hier && hier_pays(nscen)) TG_TRY(have_hier(nscen, use_dem_scen, &on));
   if (!on) {
     const int rc = ensure_legacy(S_cap);
     if (rc != TAPGPU_OK) {  // (the next call starts from its own number of scenarios)
@@ -363,15 +363,29 @@ int Ctx::choose_paths(int nscen) {
   return TAPGPU_OK;
 }
 
-// Whether the hierarchy's buffers for nscen scenarios are there, or could be made.
-bool Ctx::have_hier(int nscen) {
-  if (hier_cap >= nscen) return true;
-  if (gexec) cudaGraphExecDestroy(gexec);
-  gexec = nullptr;
-  if (ensure_hier(nscen) == TAPGPU_OK) return true;
-  cudaGetLastError();
-  release_hier();
-  return false;
+// The hierarchy's buffers and demand table for nscen scenarios; *there stays false
+// where there is no room for them.
+int Ctx::have_hier(int nscen, bool own_demand, bool* there) {
+  // (the scenarios share the base demand: one row)
+  unsigned long long** dem = own_demand ? &h_sc_dem : &h_dem;
+  const long long* q = own_demand ? sc_od_q : od_q;
+  const int rows = own_demand ? nscen : 1;
+  if (hier_cap < nscen || !*dem) {
+    if (gexec) cudaGraphExecDestroy(gexec);
+    gexec = nullptr;
+    int rc = *dem ? TAPGPU_OK : hier_demand(q, rows, dem);
+    if (rc == TAPGPU_OK && hier_cap < nscen) rc = ensure_hier(nscen);
+    if (rc != TAPGPU_OK) {
+      release_hier();
+      if (own_demand) {
+        free_owned(this, h_sc_dem);
+        h_sc_dem = nullptr;
+      }
+      return rc == TAPGPU_ERR_ALLOC ? TAPGPU_OK : rc;
+    }
+  }
+  *there = true;
+  return TAPGPU_OK;
 }
 
 // The weight records and the label buffer of the label-correction kernels.
@@ -599,9 +613,9 @@ int Ctx::hier_plan(const HierPlan* plan, const std::vector<int>& odest, const st
   for (const auto& f : at) f(dev);
   hg.pairs = pairs;
   TG_CUDA(launch_hier_pairs(hg, nodes, static_cast<int>(p.nodes.size()), chunk_of, pairs, stream));
+  TG_CUDA(cudaStreamSynchronize(stream));  // (the copy reads blob)
   h_dests = static_cast<int>(p.dest_node.size());
   h_width = static_cast<int>(by_pos.size());
-  TG_TRY(hier_demand(od_q, 1, &h_dem));
   // first exponent: twice the largest cost of a path with the fewest links
   // from the first origin at free flow just fits
   {
@@ -628,10 +642,16 @@ int Ctx::hier_plan(const HierPlan* plan, const std::vector<int>& odest, const st
   return TAPGPU_OK;
 }
 
-// Demand by destination from the OD entries dev_q [nscen][nnz] (device).
+// Demand by destination from the OD entries dev_q [nscen][nnz] (device).  A table of
+// destinations x origins however few pairs there are (1,000 zones: 8 MB a
+// scenario, 5,000: 200 MB), so it is made once a solve or loading takes the
+// hierarchy and no larger than kHierBytes.
 int Ctx::hier_demand(const long long* dev_q, int nscen, unsigned long long** dem) {
   const size_t row = static_cast<size_t>(h_dests) * h_width;
-  if (!*dem) TG_TRY(alloc_n(dem, row * nscen));
+  if (!*dem) {
+    if (row * nscen > kHierBytes / sizeof(unsigned long long)) return TAPGPU_ERR_ALLOC;
+    TG_TRY(alloc_n(dem, row * nscen));
+  }
   TG_CUDA(cudaMemsetAsync(*dem, 0, sizeof(unsigned long long) * row * nscen, stream));
   TG_CUDA(launch_hier_demand(od_ptr, h_od_dest, dev_q, nnz, nscen, Z, h_column, *dem, h_width,
                              static_cast<long long>(row), dem != &h_dem, stream));
@@ -1556,9 +1576,9 @@ int tapgpu_solve_begin(tapgpu_ctx* ctx, int max_iters, double target_relgap, con
   Ctx* c = ctx->c;
   TG_CUDA(cudaSetDevice(c->device));
   TG_TRY(c->ensure_scenarios(1));
-  TG_TRY(c->choose_paths(1));
   c->use_dem_scen = false;
   c->use_link_scen = false;
+  TG_TRY(c->choose_paths(1));
   TG_CUDA(cudaMemcpy(c->cap, c->h_cap.data(), sizeof(double) * c->M, cudaMemcpyHostToDevice));
   std::vector<int> one{0};
   TG_CUDA(cudaMemcpyAsync(c->scen_list, one.data(), sizeof(int), cudaMemcpyHostToDevice, c->stream));
@@ -1735,9 +1755,9 @@ int tapgpu_solve_scenarios(tapgpu_ctx* ctx, int num_scen, const int64_t* scen_pt
   }
   TG_CUDA(cudaSetDevice(c->device));
   TG_TRY(c->ensure_scenarios(num_scen));
-  TG_TRY(c->choose_paths(num_scen));
   c->use_dem_scen = c->dem_scen == num_scen;
   c->use_link_scen = c->link_scen == num_scen;
+  TG_TRY(c->choose_paths(num_scen));
   c->last_nscen = num_scen;
   // capacities of every scenario, made on the device from the base row and
   // the edits; the host finds each scenario's smallest positive capacity
@@ -1915,7 +1935,7 @@ int tapgpu_set_scenario_demand(tapgpu_ctx* ctx, int num_scen, const double* dema
     TG_CUDA(cudaMemcpy(c->od_q, oq.data(), sizeof(long long) * nnz, cudaMemcpyHostToDevice));
     c->scale_bits = bits;
     c->inv_scale = std::ldexp(1.0, -bits);
-    if (c->hier) TG_TRY(c->hier_demand(c->od_q, 1, &c->h_dem));
+    if (c->h_dem) TG_TRY(c->hier_demand(c->od_q, 1, &c->h_dem));
   }
   const double scale = std::ldexp(1.0, c->scale_bits);
   std::vector<long long> q(static_cast<size_t>(num_scen) * nnz);
@@ -1924,7 +1944,6 @@ int tapgpu_set_scenario_demand(tapgpu_ctx* ctx, int num_scen, const double* dema
   TG_TRY(c->alloc_n(&c->sc_total, static_cast<size_t>(num_scen)));
   TG_CUDA(cudaMemcpy(c->sc_od_q, q.data(), sizeof(long long) * q.size(), cudaMemcpyHostToDevice));
   TG_CUDA(cudaMemcpy(c->sc_total, totals.data(), sizeof(double) * num_scen, cudaMemcpyHostToDevice));
-  if (c->hier) TG_TRY(c->hier_demand(c->sc_od_q, num_scen, &c->h_sc_dem));
   c->dem_scen = num_scen;
   return TAPGPU_OK;
 }
@@ -2233,8 +2252,9 @@ int tapgpu_aon(tapgpu_ctx* ctx, const double* weights, double* volume) {
   TG_TRY(to_device_weights(c, weights, w));
   TG_CUDA(cudaMemsetAsync(c->api_yfx, 0, sizeof(unsigned long long) * c->M, c->stream));
   TG_CUDA(cudaMemsetAsync(c->err, 0, sizeof(int), c->stream));
-  bool loaded = false;
-  if (c->hier && c->hier_pays(1) && c->have_hier(1)) {
+  bool swept = false, loaded = false;
+  if (c->hier && c->hier_pays(1)) TG_TRY(c->have_hier(1, false, &swept));
+  if (swept) {
     TG_TRY(c->hier_load_api(&loaded));
     if (!loaded)
       TG_CUDA(cudaMemsetAsync(c->api_yfx, 0, sizeof(unsigned long long) * c->M, c->stream));

@@ -1,8 +1,8 @@
 // solver.cuh - host-side solver context behind the tapgpu_* C ABI.
 #pragma once
-#include <algorithm>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -275,7 +275,7 @@ struct Ctx {
   int hier_demand(const long long* dev_q, int nscen, unsigned long long** dem);
   void release_hier();
   int ensure_hier(int S);
-  bool have_hier(int nscen);
+  int have_hier(int nscen, bool own_demand, bool* there);
   bool hier_pays(int nscen, int levels, double relaxations, int arcs) const;
   bool hier_pays(int nscen) const {
     return hier_pays(nscen, static_cast<int>(h_tile_ptr.size()) - 1, hier_relaxations, hg.arcs);
