@@ -3,6 +3,7 @@
 #include "hierarchy.h"
 
 #include <algorithm>
+#include <cmath>
 #include <numeric>
 
 namespace tapgpu {
@@ -12,7 +13,10 @@ namespace {
 // Minimum-degree order on the quotient graph with element absorption,
 // approximate external degrees and merging of indistinguishable nodes (the
 // method of Amestoy, Davis and Duff 1996).  Nodes marked `early` are
-// eliminated before all others.  False when the fill exceeds max_arcs.
+// eliminated before all others; hubs, with more than 10 sqrt(n) neighbours, come
+// last and are left out of the others' degrees, as that method has it: else every
+// leaf of a hub goes through all of them (a star of 50,000 leaves 1.5 s, of
+// 100,000 5.6 s; so 21 and 36 ms).  False when the fill exceeds max_arcs.
 class MinDegree {
  public:
   MinDegree(int n, const std::vector<int>& ptr, const std::vector<int>& adj,
@@ -20,8 +24,19 @@ class MinDegree {
       : n_(n), early_(early), max_arcs_(max_arcs), vars_(n), elems_(n), members_(n), nv_(n, 1),
         deg_(n), state_(n, kVar), mark_(n, 0), w_(n, 0), prev_(n, -1), next_(n, -1),
         head_(2 * static_cast<size_t>(n) + 2, -1), hash_(n, 0), chain_(n, -1) {
+    const int most = std::max(16, static_cast<int>(10.0 * std::sqrt(static_cast<double>(n))));
+    for (int v = 0; v < n; ++v)
+      if (!early[v] && ptr[v + 1] - ptr[v] > most) {
+        state_[v] = kDead;
+        hubs_.push_back(v);
+      }
+    std::stable_sort(hubs_.begin(), hubs_.end(),
+                     [&](int a, int b) { return ptr[a + 1] - ptr[a] < ptr[b + 1] - ptr[b]; });
     for (int v = 0; v < n; ++v) {
-      vars_[v].assign(adj.begin() + ptr[v], adj.begin() + ptr[v + 1]);
+      if (state_[v] != kVar) continue;
+      vars_[v].reserve(ptr[v + 1] - ptr[v]);
+      for (int i = ptr[v]; i < ptr[v + 1]; ++i)
+        if (state_[adj[i]] == kVar) vars_[v].push_back(adj[i]);
       deg_[v] = static_cast<int>(vars_[v].size());
       insert(v);
     }
@@ -31,7 +46,7 @@ class MinDegree {
     order.clear();
     order.reserve(n_);
     int stamp = 0, wstamp = 1;
-    int lo = 0, left = n_;
+    int lo = 0, left = n_ - static_cast<int>(hubs_.size());
     std::vector<int> lp, dense_hash;
     double fill = 0;
     while (left > 0) {
@@ -158,6 +173,7 @@ class MinDegree {
       deg_[p] = weight;
       if (lp.empty()) state_[p] = kDead;
     }
+    order.insert(order.end(), hubs_.begin(), hubs_.end());
     return true;
   }
 
@@ -199,7 +215,7 @@ class MinDegree {
   const std::vector<char>& early_;
   double max_arcs_;
   std::vector<std::vector<int>> vars_, elems_, members_;
-  std::vector<int> nv_, deg_;
+  std::vector<int> nv_, deg_, hubs_;
   std::vector<char> state_;
   std::vector<int> mark_, w_, prev_, next_;
   std::vector<int> head_;
