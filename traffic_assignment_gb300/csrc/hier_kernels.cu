@@ -1678,14 +1678,15 @@ cudaError_t launch_hier_sweep(const HierArgs& a, int num_sms, cudaStream_t s) {
 
 // demand by destination: [row][dest][width] (all ones: positive but below the
 // fixed point)
-__global__ void k_hier_demand(const int* od_ptr, const int* od_dest, const long long* q, long long nnz,
-                              int origins, const int* column, Int* out, int width,
-                              long long stride, bool scenarios, bool below) {
+__global__ void k_hier_demand(const int* od_ptr, const int* od_dest, const double* od_dem,
+                              const int* dest_of, const long long* q, long long nnz, int origins,
+                              const int* column, Int* out, int width, long long stride,
+                              bool scenarios, bool below) {
   const int s = blockIdx.y;
   for (int o = blockIdx.x; o < origins; o += gridDim.x) {
     for (int j = od_ptr[o] + threadIdx.x; j < od_ptr[o + 1]; j += blockDim.x) {
-      const int dest = od_dest[j];
-      if (dest < 0) continue;
+      if (!(od_dem[j] > 0) || od_dest[j] == o + 1) continue;
+      const int dest = dest_of[od_dest[j]];
       const Int x = static_cast<Int>(q[static_cast<size_t>(s) * nnz + j]);
       if (x == 0 && scenarios) continue;  // a demand scenario removed this pair
       Int* p = out + static_cast<size_t>(s) * stride + static_cast<size_t>(dest) * width + column[o];
@@ -1696,14 +1697,14 @@ __global__ void k_hier_demand(const int* od_ptr, const int* od_dest, const long 
   }
 }
 
-cudaError_t launch_hier_demand(const int* od_ptr, const int* od_dest, const long long* q,
-                               long long nnz, int nscen, int origins, const int* column,
-                               unsigned long long* out, int width, long long stride, bool scenarios,
-                               cudaStream_t s) {
+cudaError_t launch_hier_demand(const int* od_ptr, const int* od_dest, const double* od_dem,
+                               const int* dest_of, const long long* q, long long nnz, int nscen,
+                               int origins, const int* column, unsigned long long* out, int width,
+                               long long stride, bool scenarios, cudaStream_t s) {
   const dim3 grid(std::min(origins, 1024), nscen);
   for (int below = 0; below < 2; ++below)
-    k_hier_demand<<<grid, 256, 0, s>>>(od_ptr, od_dest, q, nnz, origins, column, out, width, stride,
-                                       scenarios, below != 0);
+    k_hier_demand<<<grid, 256, 0, s>>>(od_ptr, od_dest, od_dem, dest_of, q, nnz, origins, column, out,
+                                       width, stride, scenarios, below != 0);
   return cudaGetLastError();
 }
 

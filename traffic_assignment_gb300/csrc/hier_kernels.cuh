@@ -85,12 +85,12 @@ cudaError_t launch_hier_eliminate(const HierArgs& a, int num_levels,
                                   const int* tile_ptr, cudaStream_t s);
 cudaError_t launch_hier_climb(const HierArgs& a, cudaStream_t s);
 cudaError_t launch_hier_sweep(const HierArgs& a, int num_sms, cudaStream_t s);
-// demand by destination from the OD entries q [nscen][nnz] (od_dest: destination
-// index or -1), `out` zero before
-cudaError_t launch_hier_demand(const int* od_ptr, const int* od_dest, const long long* q,
-                               long long nnz, int nscen, int origins, const int* column,
-                               unsigned long long* out, int width, long long stride, bool scenarios,
-                               cudaStream_t s);
+// demand by destination from the OD entries q [nscen][nnz] of the pairs of two nodes
+// with base demand od_dem (dest_of: destination index of a node), `out` zero before
+cudaError_t launch_hier_demand(const int* od_ptr, const int* od_dest, const double* od_dem,
+                               const int* dest_of, const long long* q, long long nnz, int nscen,
+                               int origins, const int* column, unsigned long long* out, int width,
+                               long long stride, bool scenarios, cudaStream_t s);
 cudaError_t launch_hier_load(const HierArgs& a, int num_sms, cudaStream_t s);
 
 }  // namespace tapgpu

@@ -20,8 +20,8 @@ namespace {
 class MinDegree {
  public:
   MinDegree(int n, const std::vector<int>& ptr, const std::vector<int>& adj,
-            const std::vector<char>& early, double max_arcs)
-      : n_(n), early_(early), max_arcs_(max_arcs), vars_(n), elems_(n), members_(n), nv_(n, 1),
+            const std::vector<char>& early, double max_arcs, const std::atomic<bool>* stop)
+      : n_(n), early_(early), max_arcs_(max_arcs), stop_(stop), vars_(n), elems_(n), members_(n), nv_(n, 1),
         deg_(n), state_(n, kVar), mark_(n, 0), w_(n, 0), prev_(n, -1), next_(n, -1),
         head_(2 * static_cast<size_t>(n) + 2, -1), hash_(n, 0), chain_(n, -1) {
     const int most = std::max(16, static_cast<int>(10.0 * std::sqrt(static_cast<double>(n))));
@@ -77,7 +77,7 @@ class MinDegree {
       left -= nv_[p];
       emit(p, order);
       fill += static_cast<double>(nv_[p]) * (weight + 0.5 * (nv_[p] - 1));
-      if (fill > max_arcs_) return false;
+      if (fill > max_arcs_ || (stop_ && *stop_)) return false;
       // |L_e \ L_p| of every element next to L_p
       const int base = wstamp;
       for (int v : lp)
@@ -214,6 +214,7 @@ class MinDegree {
   int n_;
   const std::vector<char>& early_;
   double max_arcs_;
+  const std::atomic<bool>* stop_;
   std::vector<std::vector<int>> vars_, elems_, members_;
   std::vector<int> nv_, deg_, hubs_;
   std::vector<char> state_;
@@ -228,7 +229,7 @@ class MinDegree {
 
 bool hier_build(int n, int m, const int* tail, const int* head, int first_thru,
                 const std::vector<char>& dests, double max_arcs, double max_relaxations,
-                HierPlan& out) {
+                HierPlan& out, const std::atomic<bool>* stop) {
   out = HierPlan();
   out.n = n;
   // undirected neighbours, each once
@@ -260,7 +261,7 @@ bool hier_build(int n, int m, const int* tail, const int* head, int first_thru,
   std::vector<char> early(n, 0);
   for (int v = 0; v < n && v < first_thru; ++v) early[v] = 1;
   std::vector<int> order;
-  if (!MinDegree(n, ptr, adj, early, max_arcs).run(order)) return false;
+  if (!MinDegree(n, ptr, adj, early, max_arcs, stop).run(order)) return false;
 
   // elimination tree of that order, then its postorder
   std::vector<int> rank(n), parent(n, -1);
@@ -341,7 +342,7 @@ bool hier_build(int n, int m, const int* tail, const int* head, int first_thru,
           }
         }
       sptr[j + 1] = static_cast<int64_t>(st.size());
-      if (static_cast<double>(st.size()) > max_arcs) return false;
+      if (static_cast<double>(st.size()) > max_arcs || (stop && *stop)) return false;
       if (par[j] >= 0) {
         older[j] = last_child[par[j]];
         last_child[par[j]] = j;

@@ -24,6 +24,7 @@
 // only): the way down from an upper neighbour to the row that may pass later
 // nodes of the chunk, so that the rows of a chunk need only U's labels.
 #pragma once
+#include <atomic>
 #include <cstdint>
 #include <vector>
 
@@ -138,9 +139,9 @@ struct HierPlan {
 // tail -> head.  Nodes below first_thru are not passed through; dests marks
 // the nodes with demand.  Returns false when the hierarchy does not suit the
 // network: links between two nodes that are not passed through, or more arcs
-// or elimination work than the limits allow.
+// or elimination work than the limits allow; and soon after *stop is set.
 bool hier_build(int n, int m, const int* tail, const int* head, int first_thru,
                 const std::vector<char>& dests, double max_arcs, double max_relaxations,
-                HierPlan& out);
+                HierPlan& out, const std::atomic<bool>* stop = nullptr);
 
 }  // namespace tapgpu

@@ -4,11 +4,13 @@
 #include "solver.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <functional>
+#include <future>
 #include <limits>
 #include <memory>
 #include <numeric>
@@ -41,6 +43,7 @@ void set_message(const std::string& m) { g_message = m; }
   } while (0)
 
 Ctx::~Ctx() {
+  builder.reset();  // (its thread reads the context)
   if (gexec) cudaGraphExecDestroy(gexec);
   for (cudaEvent_t e : ev_pool) cudaEventDestroy(e);
   if (stream) cudaStreamDestroy(stream);
@@ -346,6 +349,7 @@ bool Ctx::hier_pays(int nscen, int levels, double relaxations, int arcs) const {
 
 // The path kernels of the next iterations of nscen scenarios, and their buffers.
 int Ctx::choose_paths(int nscen) {
+  TG_TRY(take_plan());
   bool on = false;  // (no room: the label-correction kernels)
   if (hier && hier_pays(nscen)) TG_TRY(have_hier(nscen, use_dem_scen, &on));
   if (!on) {
@@ -459,25 +463,26 @@ int Ctx::alloc_records(int S) {
 // elimination hierarchy
 // ---------------------------------------------------------------------------
 
-// The host plan, made by a thread of its own while the context is set up
-// (10,000 nodes: it takes 9 ms, the setup 5 ms longer).
+// The host plan and its image for the device, made by a thread of its own from
+// the context's setup on; the first solve or loading waits for it (trees alone
+// never do, and without demand it is not started).  Setup, and setup with a first
+// solve of two iterations, ms: 10,000 nodes 9.3 and 17.0, 100,000 nodes 20 and
+// 144; with the setup waiting for the plan 14.8 and 19.4, 120 and 144; without a
+// plan 9.4 and 14.7, 20 and 89.
 class HierBuilder {
  public:
-  // the network in link order; dem: the caller's demand (origins 1..Z)
-  HierBuilder(const Ctx& c, const tapgpu_demand* dem) {
-    if (!wanted(c)) return;
-    auto work = [this, &c, dem] {
+  // (c has its network; dem is the caller's, see wait_read)
+  HierBuilder(Ctx& c, const tapgpu_demand& dem) : dests_(c.n1, 0) {
+    auto work = [this, &c, &dem] {
+      each_pair(c, dem, [this](int64_t d) {
+        dests_[d] = 1;
+        return false;
+      });
+      read_.set_value();
       try {
-        std::vector<char> dests(c.n1, 0);
-        for (int o = 1; dem && o <= c.Z; ++o)
-          for (int64_t i = dem->od_ptr[o]; i < dem->od_ptr[o + 1]; ++i) {
-            const int64_t d = dem->od_dest[i];
-            if (d < 0 || d >= c.n1) return;  // (reported when it is loaded)
-            if (dem->od_demand[i] > 0 && d != o) dests[d] = 1;
-          }
-        built_ = hier_build(c.n1, c.M, c.h_tail.data(), c.h_head.data(), c.F, dests, 80.0 * c.n1,
-                            1e11, plan_);
+        make(c);
       } catch (const std::bad_alloc&) {
+        made_ = false;
       }
     };
     try {
@@ -486,109 +491,106 @@ class HierBuilder {
       work();
     }
   }
-  ~HierBuilder() { wait(); }
-  const HierPlan* wait() {
+  ~HierBuilder() {
+    stop_ = true;
     if (thread_.joinable()) thread_.join();
-    return built_ ? &plan_ : nullptr;
   }
+  // FP64 paths (integer labels break near-ties as exact sums do, which FP64
+  // sums do too; the FP32 sums' ties fall otherwise) with demand between two
+  // nodes.  A caller's choice of a label-correction kernel or of its shape
+  // stands; networks small enough for the edge-list sweeps keep them.
+  static bool wanted(const Ctx& c, const tapgpu_demand* dem) {
+    const tapgpu_options& o = c.opt;
+    return c.fp64 && dem && (c.n1 > kSmallNet || c.M > kSmallNet) &&
+           !(o.sssp_variant || o.sssp_block || o.aon_block || o.nf_delta > 0 || o.global_scratch ||
+             o.chunk_tasks || o.sssp_ctas_per_sm || o.aon_ctas_per_sm) &&
+           each_pair(c, *dem, [](int64_t) { return true; });
+  }
+  // the caller's demand has been read
+  void wait_read() { read_.get_future().wait(); }
+  int finish(Ctx& c);
 
  private:
-  // FP64 paths (integer labels break near-ties as exact sums do, which FP64
-  // sums do too; the FP32 sums' ties fall otherwise).  A caller's choice of a
-  // label-correction kernel or of its shape stands; networks small enough for
-  // the edge-list sweeps keep them.
-  static bool wanted(const Ctx& c) {
-    const tapgpu_options& o = c.opt;
-    return c.fp64 && c.Z >= 1 && (c.n1 > kSmallNet || c.M > kSmallNet) &&
-           !(o.sssp_variant || o.sssp_block || o.aon_block || o.nf_delta > 0 || o.global_scratch ||
-             o.chunk_tasks || o.sssp_ctas_per_sm || o.aon_ctas_per_sm);
+  // fn(destination) of the pairs of two nodes with demand, until it returns true
+  template <class Fn>
+  static bool each_pair(const Ctx& c, const tapgpu_demand& dem, Fn fn) {
+    for (int64_t o = 1; o <= c.Z; ++o)
+      for (int64_t i = dem.od_ptr[o]; i < dem.od_ptr[o + 1]; ++i)
+        if (dem.od_demand[i] > 0 && dem.od_dest[i] != o && fn(dem.od_dest[i])) return true;
+    return false;
   }
+  void make(Ctx& c);
 
   HierPlan plan_;
-  bool built_ = false;
+  std::vector<char> dests_;
+  std::promise<void> read_;
+  std::atomic<bool> stop_{false};
+  bool made_ = false;
   std::thread thread_;
+  // one allocation and one copy for all of the plan's arrays
+  std::vector<unsigned char> blob_;
+  std::vector<std::function<void(unsigned char*)>> at_;
+  HierPlan::Node* nodes_ = nullptr;
+  int* chunk_of_ = nullptr;
+  int u_exp0_ = 0, width_ = 0;
 };
 
-// The plan on the device, where the hierarchy can pay.  (odest, optr, odem: the
-// demand as a CSR over origin slots)
-int Ctx::hier_plan(const HierPlan* plan, const std::vector<int>& odest, const std::vector<int>& optr,
-                   const std::vector<double>& odem) {
-  hier = false;
-  if (!plan) return TAPGPU_OK;
-  const HierPlan& p = *plan;
-  if (hier_climb_smem(p.climb) > kHierMaxClimb || p.climb > 0xffff) return TAPGPU_OK;
-  if (!hier_pays(4096, p.num_levels, p.relaxations, p.arcs)) return TAPGPU_OK;
-  std::vector<int> odpos(odest.size(), -1);
-  for (int o = 0; o < Z; ++o)
-    for (int i = optr[o]; i < optr[o + 1]; ++i)
-      if (odem[i] > 0 && odest[i] != o + 1) odpos[i] = odest[i];
+// (reads the context's network, notes where its pointers to the device go)
+void HierBuilder::make(Ctx& c) {
+  HierPlan& p = plan_;
+  const int n1 = c.n1, Z = c.Z, M = c.M;
+  if (!hier_build(n1, M, c.h_tail.data(), c.h_head.data(), c.F, dests_, 80.0 * n1, 1e11, p, &stop_))
+    return;
+  if (hier_climb_smem(p.climb) > kHierMaxClimb || p.climb > 0xffff) return;
   std::vector<int> dest_of(n1, -1);
   for (size_t i = 0; i < p.dest_node.size(); ++i) dest_of[p.dest_node[i]] = static_cast<int>(i);
-  for (auto& x : odpos)
-    if (x >= 0) x = dest_of[x];
-
-  hier_relaxations = p.relaxations;
-  hg.n = p.n;
-  hg.arcs = p.arcs;
-  hg.climb = p.climb;
-  hg.num_elims = static_cast<int>(p.elims.size());
-  hg.num_marks = static_cast<int>(p.marks.size());
-  h_tile_ptr = p.tile_ptr;
-  hg.top_rows = p.top_rows;
-  hg.top_levels = p.top_levels;
-  hg.num_subs = static_cast<int>(p.subs.size());
   std::vector<unsigned short> iclimb(p.idx.size()), aclimb(static_cast<size_t>(p.arcs), 0);
   for (size_t i = 0; i < p.idx.size(); ++i) {
-    const HierChunk& c = p.chunks[p.chunk_of[p.idx[i]]];
-    iclimb[i] = static_cast<unsigned short>(c.coff + p.idx[i] - c.first);
+    const HierChunk& k = p.chunks[p.chunk_of[p.idx[i]]];
+    iclimb[i] = static_cast<unsigned short>(k.coff + p.idx[i] - k.first);
   }
-  for (const auto& c : p.chunks)
-    for (int i = 0; i < c.k; ++i)
-      std::fill_n(aclimb.begin() + c.woff + i * c.ld, c.ld, static_cast<unsigned short>(c.coff + i));
-  // one allocation and one copy for all of it
-  std::vector<unsigned char> blob;
-  std::vector<std::function<void(unsigned char*)>> at;
+  for (const auto& k : p.chunks)
+    for (int i = 0; i < k.k; ++i)
+      std::fill_n(aclimb.begin() + k.woff + i * k.ld, k.ld, static_cast<unsigned short>(k.coff + i));
   auto put = [&](auto** dst, const auto& v) {
-    at.push_back([dst, off = blob.size()](unsigned char* base) {
+    at_.push_back([dst, off = blob_.size()](unsigned char* base) {
       *dst = reinterpret_cast<typename std::remove_reference<decltype(*dst)>::type>(base + off);
     });
     const auto* q = reinterpret_cast<const unsigned char*>(v.data());
-    blob.insert(blob.end(), q, q + v.size() * sizeof(v[0]));
-    blob.resize((blob.size() + 255) / 256 * 256);
+    blob_.insert(blob_.end(), q, q + v.size() * sizeof(v[0]));
+    blob_.resize((blob_.size() + 255) / 256 * 256);
   };
-  blob.reserve(sizeof(int) * (8 * static_cast<size_t>(p.arcs) + 8 * p.idx.size() + p.rel.size() +
-                              64 * static_cast<size_t>(n1)));
-  put(&hg.chunks, p.chunks);
-  put(&hg.shut, p.shut);
-  put(&hg.idx, p.idx);
-  put(&hg.idx_climb, iclimb);
-  put(&hg.arc_climb, aclimb);
-  put(&hg.tgt_base, p.tgt_base);
-  put(&hg.tgt_rel, p.tgt_rel);
-  put(&hg.rel, p.rel);
-  put(&hg.arc_link, p.arc_link);
-  put(&hg.link_arc, p.link_arc);
-  put(&hg.link_next, p.link_next);
-  put(&hg.elims, p.elims);
-  put(&hg.elim_pair, p.elim_pair);
-  put(&hg.elim_close, p.elim_close);
-  HierPlan::Node* nodes = nullptr;
-  int* chunk_of = nullptr;
-  put(&nodes, p.nodes);
-  put(&chunk_of, p.chunk_of);
-  put(&hg.tiles, p.tiles);
-  put(&hg.marks, p.marks);
-  put(&hg.tops, p.tops);
-  put(&hg.top_uidx, p.top_uidx);
-  put(&hg.top_dest, p.top_dest);
-  put(&hg.job_ptr, p.job_ptr);
-  put(&hg.jobs, p.jobs);
-  put(&hg.subs, p.subs);
-  put(&hg.sub_ext, p.sub_ext);
-  put(&hg.sub_rows, p.sub_rows);
-  put(&hg.sub_slot, p.sub_slot);
-  put(&hg.sub_ids, p.sub_ids);
-  put(&h_od_dest, odpos);
+  blob_.reserve(sizeof(int) * (8 * static_cast<size_t>(p.arcs) + 8 * p.idx.size() + p.rel.size() +
+                               64 * static_cast<size_t>(n1)));
+  put(&c.hg.chunks, p.chunks);
+  put(&c.hg.shut, p.shut);
+  put(&c.hg.idx, p.idx);
+  put(&c.hg.idx_climb, iclimb);
+  put(&c.hg.arc_climb, aclimb);
+  put(&c.hg.tgt_base, p.tgt_base);
+  put(&c.hg.tgt_rel, p.tgt_rel);
+  put(&c.hg.rel, p.rel);
+  put(&c.hg.arc_link, p.arc_link);
+  put(&c.hg.link_arc, p.link_arc);
+  put(&c.hg.link_next, p.link_next);
+  put(&c.hg.elims, p.elims);
+  put(&c.hg.elim_pair, p.elim_pair);
+  put(&c.hg.elim_close, p.elim_close);
+  put(&nodes_, p.nodes);
+  put(&chunk_of_, p.chunk_of);
+  put(&c.hg.tiles, p.tiles);
+  put(&c.hg.marks, p.marks);
+  put(&c.hg.tops, p.tops);
+  put(&c.hg.top_uidx, p.top_uidx);
+  put(&c.hg.top_dest, p.top_dest);
+  put(&c.hg.job_ptr, p.job_ptr);
+  put(&c.hg.jobs, p.jobs);
+  put(&c.hg.subs, p.subs);
+  put(&c.hg.sub_ext, p.sub_ext);
+  put(&c.hg.sub_rows, p.sub_rows);
+  put(&c.hg.sub_slot, p.sub_slot);
+  put(&c.hg.sub_ids, p.sub_ids);
+  put(&c.h_dest_of, dest_of);
   // origins in position order: neighbours in the network share a group
   std::vector<int> opos(Z), by_pos(Z), column(Z), chain_ptr(Z + 1, 0), chain;
   for (int o = 0; o < Z; ++o) opos[o] = p.pos[o + 1];
@@ -596,50 +598,79 @@ int Ctx::hier_plan(const HierPlan* plan, const std::vector<int>& odest, const st
   std::sort(by_pos.begin(), by_pos.end(), [&](int a, int b) { return opos[a] < opos[b]; });
   for (int i = 0; i < Z; ++i) column[by_pos[i]] = i;
   for (int o = 0; o < Z; ++o) {
-    for (int c = p.chunk_of[opos[o]]; c >= 0; c = p.chunks[c].parent) chain.push_back(c);
+    for (int k = p.chunk_of[opos[o]]; k >= 0; k = p.chunks[k].parent) chain.push_back(k);
     chain_ptr[o + 1] = static_cast<int>(chain.size());
   }
   while (by_pos.size() % kHierWidth) by_pos.push_back(-1);
-  put(&h_opos, opos);
-  put(&h_group, by_pos);
-  put(&h_column, column);
-  put(&h_chain_ptr, chain_ptr);
-  put(&h_chain, chain);
-  unsigned char* dev = nullptr;
-  HierPlan::Pair* pairs = nullptr;
-  TG_TRY(alloc_n(&dev, blob.size()));
-  TG_TRY(alloc_n(&pairs, static_cast<size_t>(p.num_pairs)));
-  TG_CUDA(cudaMemcpyAsync(dev, blob.data(), blob.size(), cudaMemcpyHostToDevice, stream));
-  for (const auto& f : at) f(dev);
-  hg.pairs = pairs;
-  TG_CUDA(launch_hier_pairs(hg, nodes, static_cast<int>(p.nodes.size()), chunk_of, pairs, stream));
-  TG_CUDA(cudaStreamSynchronize(stream));  // (the copy reads blob)
-  h_dests = static_cast<int>(p.dest_node.size());
-  h_width = static_cast<int>(by_pos.size());
+  put(&c.h_opos, opos);
+  put(&c.h_group, by_pos);
+  put(&c.h_column, column);
+  put(&c.h_chain_ptr, chain_ptr);
+  put(&c.h_chain, chain);
+  width_ = static_cast<int>(by_pos.size());
   // first exponent: twice the largest cost of a path with the fewest links
   // from the first origin at free flow just fits
-  {
-    std::vector<int> rp(n1 + 1, 0), queue{1};
-    for (int k = 0; k < M; ++k) ++rp[h_tail[k] + 1];
-    for (int v = 0; v < n1; ++v) rp[v + 1] += rp[v];
-    std::vector<double> far(n1, -1.0);
-    far[1] = 0.0;
-    double most = 0.0;
-    for (size_t i = 0; i < queue.size(); ++i) {
-      const int v = queue[i];
-      most = std::max(most, far[v]);
-      for (int k = rp[v]; k < rp[v + 1]; ++k)
-        if (far[h_head[k]] < 0) {
-          far[h_head[k]] = far[v] + h_fft[k];
-          queue.push_back(h_head[k]);
-        }
-    }
-    int e = 0;
-    if (most > 0) e = 59 - static_cast<int>(std::ceil(std::log2(most))) - 1;
-    u_exp0 = std::max(-900, std::min(900, e));
+  std::vector<int> rp(n1 + 1, 0), queue{1};
+  for (int k = 0; k < M; ++k) ++rp[c.h_tail[k] + 1];
+  for (int v = 0; v < n1; ++v) rp[v + 1] += rp[v];
+  std::vector<double> far(n1, -1.0);
+  far[1] = 0.0;
+  double most = 0.0;
+  for (size_t i = 0; i < queue.size(); ++i) {
+    const int v = queue[i];
+    most = std::max(most, far[v]);
+    for (int k = rp[v]; k < rp[v + 1]; ++k)
+      if (far[c.h_head[k]] < 0) {
+        far[c.h_head[k]] = far[v] + c.h_fft[k];
+        queue.push_back(c.h_head[k]);
+      }
   }
-  hier = true;
+  int e = 0;
+  if (most > 0) e = 59 - static_cast<int>(std::ceil(std::log2(most))) - 1;
+  u_exp0_ = std::max(-900, std::min(900, e));
+  made_ = true;
+}
+
+// The plan on the device, where the hierarchy can pay and there is room for it.
+int HierBuilder::finish(Ctx& c) {
+  if (thread_.joinable()) thread_.join();
+  const HierPlan& p = plan_;
+  if (!made_ || !c.hier_pays(4096, p.num_levels, p.relaxations, p.arcs)) return TAPGPU_OK;
+  unsigned char* dev = nullptr;
+  HierPlan::Pair* pairs = nullptr;
+  if (c.alloc_n(&dev, blob_.size()) != TAPGPU_OK ||
+      c.alloc_n(&pairs, static_cast<size_t>(p.num_pairs)) != TAPGPU_OK) {
+    free_owned(&c, dev);
+    return TAPGPU_OK;
+  }
+  TG_CUDA(cudaMemcpyAsync(dev, blob_.data(), blob_.size(), cudaMemcpyHostToDevice, c.stream));
+  for (const auto& f : at_) f(dev);
+  HierGraph& hg = c.hg;
+  hg.n = p.n;
+  hg.arcs = p.arcs;
+  hg.climb = p.climb;
+  hg.num_elims = static_cast<int>(p.elims.size());
+  hg.num_marks = static_cast<int>(p.marks.size());
+  hg.top_rows = p.top_rows;
+  hg.top_levels = p.top_levels;
+  hg.num_subs = static_cast<int>(p.subs.size());
+  hg.pairs = pairs;
+  TG_CUDA(launch_hier_pairs(hg, nodes_, static_cast<int>(p.nodes.size()), chunk_of_, pairs, c.stream));
+  TG_CUDA(cudaStreamSynchronize(c.stream));  // (the copy reads blob_)
+  c.hier_relaxations = p.relaxations;
+  c.h_tile_ptr = p.tile_ptr;
+  c.h_dests = static_cast<int>(p.dest_node.size());
+  c.h_width = width_;
+  c.u_exp0 = u_exp0_;
+  c.hier = true;
   return TAPGPU_OK;
+}
+
+// Waits for a plan under way.
+int Ctx::take_plan() {
+  if (!builder) return TAPGPU_OK;
+  const std::shared_ptr<HierBuilder> b = std::move(builder);
+  return b->finish(*this);
 }
 
 // Demand by destination from the OD entries dev_q [nscen][nnz] (device).  A table of
@@ -653,7 +684,7 @@ int Ctx::hier_demand(const long long* dev_q, int nscen, unsigned long long** dem
     TG_TRY(alloc_n(dem, row * nscen));
   }
   TG_CUDA(cudaMemsetAsync(*dem, 0, sizeof(unsigned long long) * row * nscen, stream));
-  TG_CUDA(launch_hier_demand(od_ptr, h_od_dest, dev_q, nnz, nscen, Z, h_column, *dem, h_width,
+  TG_CUDA(launch_hier_demand(od_ptr, od_dest, od_dem, h_dest_of, dev_q, nnz, nscen, Z, h_column, *dem, h_width,
                              static_cast<long long>(row), dem != &h_dem, stream));
   TG_CUDA(cudaStreamSynchronize(stream));
   return TAPGPU_OK;
@@ -1267,7 +1298,7 @@ static int create_impl(const tapgpu_network* net, const tapgpu_demand* dem,
     c->nf_delta = opt.nf_delta > 0 ? opt.nf_delta : (mean > 0 ? 16.0 * mean : 1.0);
   }
 
-  HierBuilder builder(*c, dem);
+  if (HierBuilder::wanted(*c, dem)) c->builder = std::make_shared<HierBuilder>(*c, *dem);
 
   std::vector<int> rp(n1 + 1, 0), ip_in(n1 + 1, 0), inl(M);
   for (int k = 0; k < M; ++k) {
@@ -1432,8 +1463,10 @@ static int create_impl(const tapgpu_network* net, const tapgpu_demand* dem,
   TG_TRY(c->alloc_n(&c->api_yfx, M));
   TG_TRY(c->ensure_scenarios(1));
   TG_CUDA(cudaMemcpy(c->cap, c->h_cap.data(), sizeof(double) * M, cudaMemcpyHostToDevice));
-  TG_TRY(c->hier_plan(builder.wait(), odest, optr, odem));
-  TG_TRY(c->choose_paths(1));
+  if (c->builder)
+    c->builder->wait_read();
+  else
+    TG_TRY(c->choose_paths(1));
   *out = guard.release();
   return TAPGPU_OK;
 }
@@ -2253,6 +2286,7 @@ int tapgpu_aon(tapgpu_ctx* ctx, const double* weights, double* volume) {
   TG_CUDA(cudaMemsetAsync(c->api_yfx, 0, sizeof(unsigned long long) * c->M, c->stream));
   TG_CUDA(cudaMemsetAsync(c->err, 0, sizeof(int), c->stream));
   bool swept = false, loaded = false;
+  TG_TRY(c->take_plan());
   if (c->hier && c->hier_pays(1)) TG_TRY(c->have_hier(1, false, &swept));
   if (swept) {
     TG_TRY(c->hier_load_api(&loaded));

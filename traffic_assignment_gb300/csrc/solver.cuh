@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -31,6 +32,8 @@ constexpr int kSpreadIters = 2;
 inline int64_t rows_at_once(int64_t rows, int n1) {
   return std::max<int64_t>(1, std::min<int64_t>(rows, (int64_t(64) << 20) / (int64_t(8) * n1)));
 }
+
+class HierBuilder;
 
 struct Ctx {
   // sizes (internal link order: sorted by (init, term))
@@ -150,7 +153,8 @@ struct Ctx {
   // elimination hierarchy (hierarchy.h): the solver's shortest paths and
   // loading where the plan suits the network; the label-correction kernels
   // otherwise, and for a scenario whose labels leave the integers' range
-  bool hier = false;             // its plan is in place
+  std::shared_ptr<HierBuilder> builder;  // makes the plan, until it is asked for
+  bool hier = false;             // the plan is in place
   bool hier_on = false;          // the iterations run on it (choose_paths)
   ScenState* api_state = nullptr;  // of a loading through the API
   int hier_cap = 0;              // scenarios that its buffers were made for
@@ -160,7 +164,7 @@ struct Ctx {
   int u_exp0 = 0;                // exponent of the first labels
   int *h_opos = nullptr, *h_group = nullptr, *h_column = nullptr;  // origins by position
   int *h_chain_ptr = nullptr, *h_chain = nullptr;
-  int* h_od_dest = nullptr;      // destination index of each OD entry or -1
+  int* h_dest_of = nullptr;      // destination index of each node or -1
   int h_dests = 0, h_width = 0;  // demand by destination: [h_dests][h_width]
   unsigned long long *h_dem = nullptr, *h_sc_dem = nullptr;
   size_t hier_bytes = kHierBytes;  // bound of the buffers below
@@ -270,8 +274,7 @@ struct Ctx {
   int enqueue_initial(int nscen, bool warm);
   int enqueue_tail(int nscen, bool records = false);
   int run_graph(int iters, int nscen);
-  int hier_plan(const HierPlan* plan, const std::vector<int>& odest, const std::vector<int>& optr,
-                const std::vector<double>& odem);
+  int take_plan();
   int hier_demand(const long long* dev_q, int nscen, unsigned long long** dem);
   void release_hier();
   int ensure_hier(int S);
