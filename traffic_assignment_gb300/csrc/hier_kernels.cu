@@ -1651,6 +1651,11 @@ cudaError_t sweep_t(const HierArgs& a, int num_sms, cudaStream_t s) {
 
 }  // namespace
 
+int hier_launches(const HierGraph& h, int num_levels) {
+  return 2 + num_levels + 2 * (h.num_elims > 0) + (h.num_marks > 0) + 2 * (h.top_levels > 0) +
+         (h.num_subs > 0) + kSplitPasses + 5;
+}
+
 size_t hier_climb_smem(int climb) {
   return (sizeof(Int) + sizeof(int)) * static_cast<size_t>(climb);
 }

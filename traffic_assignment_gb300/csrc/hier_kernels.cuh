@@ -92,5 +92,7 @@ cudaError_t launch_hier_demand(const int* od_ptr, const int* od_dest, const doub
                                int origins, const int* column, unsigned long long* out, int width,
                                long long stride, bool scenarios, cudaStream_t s);
 cudaError_t launch_hier_load(const HierArgs& a, int num_sms, cudaStream_t s);
+// kernels of one elimination, climb, sweep and loading
+int hier_launches(const HierGraph& h, int num_levels);
 
 }  // namespace tapgpu

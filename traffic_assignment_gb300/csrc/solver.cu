@@ -749,7 +749,7 @@ int Ctx::enqueue_hier(int nscen, const double* cost, long long stride, cudaEvent
     if (measuring) TG_TRY(mark(1, true));
     TG_CUDA(launch_hier_load(a, num_sms, stream));
     if (measuring) TG_TRY(mark(1, false));
-    count_launches(levels + 24);
+    count_launches(hier_launches(hg, levels));
   }
   return TAPGPU_OK;
 }
@@ -829,6 +829,7 @@ int Ctx::hier_load_api(bool* loaded) {
     TG_CUDA(launch_hier_climb(a, stream));
     TG_CUDA(launch_hier_sweep(a, num_sms, stream));
     TG_CUDA(launch_hier_load(a, num_sms, stream));
+    count_launches(hier_launches(hg, levels));
     TG_CUDA(cudaStreamSynchronize(stream));
     TG_CUDA(cudaMemcpy(&st, api_state, sizeof(st), cudaMemcpyDeviceToHost));
     if (!st.done) {
