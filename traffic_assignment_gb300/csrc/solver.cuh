@@ -234,12 +234,15 @@ struct Ctx {
   // below 2^-12 and the one block takes 20 us longer (416 nodes to relative gap
   // 1e-5, 26,000 iterations: 12,700 -> 17,200 it/s with two).
   int grid_passes() const { return ls_mode == kLsExact ? 6 : 2; }
-  // One scenario whose links make a few more blocks than there are SMs: one
-  // block per SM, its share a little longer (40,000 links: 157 blocks gave five
-  // SMs twice the FP64 work).
+  // One scenario whose links make up to two blocks per SM: one block per SM, its
+  // share longer.  Else some SMs have twice the FP64 work of the others, a step
+  // that costs as much at 1.01 as at 1.95 blocks per SM.  Line search of an
+  // iteration in FP64 mode, us, by blocks per SM: 1.01 58 -> 44, 1.25 59 -> 45, 1.5
+  // 61 -> 47, 1.8 61 -> 49, 1.95 61 -> 51 (FP32 mode 50..53 -> 39..41); at two the
+  // grid is full (68 either way).
   int step_grid(int nscen) const {
-    return nscen == 1 && ls_link_grid > num_sms && 4 * ls_link_grid < 5 * num_sms ? num_sms
-                                                                                  : ls_link_grid;
+    return nscen == 1 && ls_link_grid > num_sms && ls_link_grid < 2 * num_sms ? num_sms
+                                                                              : ls_link_grid;
   }
 
   std::vector<DevMem> owned;
