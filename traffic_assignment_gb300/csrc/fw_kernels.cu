@@ -1994,7 +1994,6 @@ constexpr int kLinkBlock = 256;
 // With from_x set, x is taken as given (warm start).
 __global__ void __launch_bounds__(kLinkBlock) k_init_flows(LinkArgs a, int from_x) {
   const int scen = scen_of(a);
-  if (a.state[scen].done > 1) return;  // paused in its first loading: nothing to start from
   const size_t off = static_cast<size_t>(scen) * a.m;
   const double* cap = a.cap + off;
   for (int k = blockIdx.x * kLinkBlock + threadIdx.x; k < a.m; k += gridDim.x * kLinkBlock) {

@@ -205,11 +205,11 @@ cudaError_t launch_aon(const PathArgs& a, bool fp64, int grid, int block, bool s
 cudaError_t launch_init_flows(const LinkArgs& a, int grid, cudaStream_t s);
 // weights = free-flow times and y_fx = 0 (first all-or-nothing)
 cudaError_t launch_set_costs(const LinkArgs& a, int grid, cudaStream_t s);
+// weights of the label-correction kernels' records from the current costs t
+cudaError_t launch_records(const LinkArgs& a, int grid, cudaStream_t s);
 // line-search passes and the step: `block` kSmallLinkBlock (networks of at
 // most kSmallNet links, FP64 work over more SMs) or kLinkBlock
 constexpr int kSmallLinkBlock = 64;
-// weights of the label-correction kernels' records from the current costs t
-cudaError_t launch_records(const LinkArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_ls_pass(const LinkArgs& a, int grid, int block, cudaStream_t s);
 cudaError_t launch_ls_rest(const LinkArgs& a, cudaStream_t s);  // passes a.pass and on
 cudaError_t launch_step(const LinkArgs& a, int grid, int block, cudaStream_t s);
@@ -226,11 +226,11 @@ cudaError_t launch_param_rows(double* rows, const double* base, int m, int nscen
 cudaError_t launch_param_rows(unsigned char* rows, const unsigned char* base, int m, int nscen,
                               const int* ptr, const int* link, const unsigned char* val, int grid,
                               cudaStream_t s);
-// rows 1 .. nscen-1 of x [nscen][m] become copies of row 0
 // the shortest-path API's results: labels in place (out of reach: DBL_MAX) and
 // predecessors as the caller's link indices (none: -1)
 cudaError_t launch_tree_rows(double* dist, size_t labels, const int* pred, const int64_t* perm,
                              int64_t* out, size_t preds, cudaStream_t s);
+// rows 1 .. nscen-1 of x [nscen][m] become copies of row 0
 cudaError_t launch_replicate_rows(double* x, int m, int nscen, int grid, cudaStream_t s);
 cudaError_t launch_fill_records(uint2* p, size_t n, uint2 val, int grid, cudaStream_t s);
 cudaError_t launch_fill_records4(uint4* p, size_t n, uint4 val, int grid, cudaStream_t s);

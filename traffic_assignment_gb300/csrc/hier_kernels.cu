@@ -1578,7 +1578,9 @@ cudaError_t launch_with(Fn fn, dim3 grid, int block, size_t smem, int cluster, b
   return cudaLaunchKernelEx(&cfg, fn, args...);
 }
 
-cudaError_t eliminate_t(const HierArgs& a, int num_levels, const int* tile_ptr, cudaStream_t s) {
+}  // namespace
+
+cudaError_t launch_hier_eliminate(const HierArgs& a, int num_levels, const int* tile_ptr, cudaStream_t s) {
   cudaError_t e = max_smem(k_hier_mark);
   if (e != cudaSuccess) return e;
   const int wb = (3 * a.h.arcs + 4 * kElimBlock - 1) / (4 * kElimBlock);
@@ -1596,7 +1598,7 @@ cudaError_t eliminate_t(const HierArgs& a, int num_levels, const int* tile_ptr, 
   return cudaGetLastError();
 }
 
-cudaError_t climb_t(const HierArgs& a, cudaStream_t s) {
+cudaError_t launch_hier_climb(const HierArgs& a, cudaStream_t s) {
   const size_t per = hier_climb_smem(a.h.climb);
   const int warps = static_cast<int>(std::max<size_t>(1, std::min<size_t>(4, kHierMaxClimb / per)));
   cudaError_t e = max_smem(k_hier_climb);
@@ -1606,7 +1608,7 @@ cudaError_t climb_t(const HierArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t descend_t(const HierArgs& a, cudaStream_t s) {
+static cudaError_t descend_t(const HierArgs& a, cudaStream_t s) {
   const size_t per = sizeof(Int) * static_cast<size_t>(a.h.climb);
   const int warps = static_cast<int>(std::max<size_t>(1, std::min<size_t>(4, kHierMaxClimb / per)));
   cudaError_t e = max_smem(k_hier_descend);
@@ -1617,14 +1619,14 @@ cudaError_t descend_t(const HierArgs& a, cudaStream_t s) {
 }
 
 template <int T>
-cudaError_t top_t(const HierArgs& a, int cluster, cudaStream_t s) {
+static cudaError_t top_t(const HierArgs& a, int cluster, cudaStream_t s) {
   const size_t smem = sizeof(TopShared<T>) * (kTopBlock / 32);
   cudaError_t e = max_smem(k_hier_top<T>);
   if (e != cudaSuccess) return e;
   return launch_with(k_hier_top<T>, dim3(a.nslots * a.groups * cluster), kTopBlock, smem, cluster, false, s, a, cluster);
 }
 
-cudaError_t sweep_t(const HierArgs& a, int num_sms, cudaStream_t s) {
+cudaError_t launch_hier_sweep(const HierArgs& a, int num_sms, cudaStream_t s) {
   const int cells = a.nslots * a.groups;
   // A group's blocks in one cluster while there are SMs for all of them (top:
   // a block fills an SM; two waves of clusters of four took 485 us for 64
@@ -1649,8 +1651,6 @@ cudaError_t sweep_t(const HierArgs& a, int num_sms, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-}  // namespace
-
 int hier_launches(const HierGraph& h, int num_levels) {
   return 2 + num_levels + 2 * (h.num_elims > 0) + (h.num_marks > 0) + 2 * (h.top_levels > 0) +
          (h.num_subs > 0) + kSplitPasses + 5;
@@ -1666,19 +1666,6 @@ cudaError_t launch_hier_pairs(const HierGraph& h, const HierPlan::Node* nodes, i
     k_hier_pairs<<<(count + kElimBlock / 32 - 1) / (kElimBlock / 32), kElimBlock, 0, s>>>(
         h, nodes, count, chunk_of, pairs);
   return cudaGetLastError();
-}
-
-cudaError_t launch_hier_eliminate(const HierArgs& a, int num_levels,
-                                  const int* tile_ptr, cudaStream_t s) {
-  return eliminate_t(a, num_levels, tile_ptr, s);
-}
-
-cudaError_t launch_hier_climb(const HierArgs& a, cudaStream_t s) {
-  return climb_t(a, s);
-}
-
-cudaError_t launch_hier_sweep(const HierArgs& a, int num_sms, cudaStream_t s) {
-  return sweep_t(a, num_sms, s);
 }
 
 // demand by destination: [row][dest][width] (all ones: positive but below the
@@ -1713,7 +1700,7 @@ cudaError_t launch_hier_demand(const int* od_ptr, const int* od_dest, const doub
   return cudaGetLastError();
 }
 
-static cudaError_t load_t(const HierArgs& a, int num_sms, cudaStream_t s) {
+cudaError_t launch_hier_load(const HierArgs& a, int num_sms, cudaStream_t s) {
   cudaError_t e = descend_t(a, s);
   if (e != cudaSuccess) return e;
   const int cb = (3 * a.h.arcs + kCollect * kElimBlock - 1) / (kCollect * kElimBlock);
@@ -1726,10 +1713,6 @@ static cudaError_t load_t(const HierArgs& a, int num_sms, cudaStream_t s) {
   k_hier_links<<<dim3((a.m + kElimBlock - 1) / kElimBlock, a.nslots), kElimBlock, 0, s>>>(a);
   k_hier_exponents<<<(a.nslots + kElimBlock - 1) / kElimBlock, kElimBlock, 0, s>>>(a);
   return cudaGetLastError();
-}
-
-cudaError_t launch_hier_load(const HierArgs& a, int num_sms, cudaStream_t s) {
-  return load_t(a, num_sms, s);
 }
 
 }  // namespace tapgpu

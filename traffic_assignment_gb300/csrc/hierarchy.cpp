@@ -349,7 +349,6 @@ bool hier_build(int n, int m, const int* tail, const int* head, int first_thru,
       }
     }
   }
-  out.real_arcs = sptr[n];
 
   // chunks
   out.chunk_of.resize(n);

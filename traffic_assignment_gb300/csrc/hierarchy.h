@@ -53,7 +53,6 @@ struct alignas(16) HierChunk {
 struct HierPlan {
   int n = 0;                      // nodes (positions)
   int arcs = 0;                   // arc slots
-  int64_t real_arcs = 0;          // without padding
   double relaxations = 0;         // triangle relaxations of one elimination
   int climb = 0;                  // climb slots (largest coff + k)
   std::vector<int> pos, node;     // node -> position and back
