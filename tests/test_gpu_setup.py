@@ -1,6 +1,8 @@
 """Contexts that may take the elimination hierarchy: set up without waiting for its
 plan, which the first solve or loading asks for."""
 
+import os
+import signal
 import time
 
 import numpy as np
@@ -61,3 +63,27 @@ def test_first_uses(built_lib):
         _, on = _on_hierarchy(s, lambda: s.solve(max_iters=2))
         assert on
         np.testing.assert_array_equal(s.flows()[0], x)
+
+
+def _threads():
+    return set(os.listdir("/proc/self/task"))
+
+
+def test_signals_are_the_callers(built_lib):
+    """The plan's thread goes on after the setup, perhaps while the caller blocks
+    signals in its own threads to wait for them: none may be delivered to it."""
+    net, dem = _net(200, 200, 150, seed=63)
+    Solver(net, dem, precision="fp64", sssp_variant="nearfar_queue").close()
+    blocked = []
+    for _ in range(3):
+        before = _threads()
+        with Solver(net, dem, precision="fp64"):
+            for t in _threads() - before:
+                try:
+                    with open(f"/proc/self/task/{t}/status") as f:
+                        mask = int(next(x for x in f if x.startswith("SigBlk")).split()[1], 16)
+                except (OSError, StopIteration):
+                    continue  # (it has ended)
+                blocked += [bool(mask >> (n - 1) & 1) for n in
+                            (signal.SIGINT, signal.SIGTERM, signal.SIGUSR1, signal.SIGUSR2)]
+    assert blocked and all(blocked)

@@ -3,6 +3,8 @@
 // CUDA graphs), and implements the tapgpu_* handle API of include/tap_gpu.h.
 #include "solver.cuh"
 
+#include <signal.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cfloat>
@@ -485,11 +487,18 @@ class HierBuilder {
         made_ = false;
       }
     };
+    // (outlives the call: the caller's signals are not for it)
+    sigset_t all, mask;
+    sigfillset(&all);
+    pthread_sigmask(SIG_SETMASK, &all, &mask);
+    bool started = true;
     try {
       thread_ = std::thread(work);
     } catch (const std::system_error&) {
-      work();
+      started = false;
     }
+    pthread_sigmask(SIG_SETMASK, &mask, nullptr);
+    if (!started) work();
   }
   ~HierBuilder() {
     stop_ = true;
