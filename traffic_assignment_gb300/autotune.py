@@ -3,8 +3,10 @@
 The fastest shortest-path kernel depends on the network (node count, degree,
 cost spread) and on how many tasks a launch holds.  ``tune`` sweeps
 
+  * the library's own choice (the elimination hierarchy for FP64 batches where
+    it pays, which any of the options below rules out),
   * the shortest-path variant: bulk-synchronous rounds, asynchronous
-    worklist, near-far, near-far with a FIFO ring (the default),
+    worklist, near-far, near-far with a FIFO ring,
   * its block size (128 .. 1024 threads),
   * the near-far phase step, as a multiple of the mean free-flow time,
   * the all-or-nothing loading block size,
@@ -74,7 +76,9 @@ def candidates(quick: bool = False, net: Optional[Network] = None) -> List[Candi
     """The sweep: every variant x block, and near-far x step scale, with the
     library's loading shape; then the loading kernel's block at the library's
     shortest-path shape (block 0: the library's choice); with a small network
-    (at most SMALL_NET nodes and links) the edge-list sweeps too."""
+    (at most SMALL_NET nodes and links) the edge-list sweeps too; first, for a
+    given network, no choice at all (10,000 nodes, 64 FP64 scenarios: the fastest
+    of the others took 4 times as long as the hierarchy)."""
     out = []
     blocks = (256, 512) if quick else (128, 256, 512, 1024)
     scales = (8.0, 16.0, 32.0) if quick else (4.0, 8.0, 16.0, 32.0, 64.0)
@@ -89,6 +93,8 @@ def candidates(quick: bool = False, net: Optional[Network] = None) -> List[Candi
                 out.append(Candidate(v, b, 16.0, 0))
     # the loading kernel's block, at the default shortest-path shape
     out.extend(Candidate("nearfar_queue", 0, 16.0, a) for a in (256, 512, 1024))
+    if net is not None:
+        out.insert(0, Candidate("default", 0, 16.0, 0))
     return out
 
 
@@ -106,8 +112,9 @@ def cache_key(net: Network, precision: str, scenarios: int, device_name: str) ->
     h = hashlib.sha1()
     for a in (net.init, net.term, net.fft, net.capacity):
         h.update(np.ascontiguousarray(a).tobytes())
+    # ("default": sweeps that did not have that candidate are not served)
     h.update(repr((net.num_nodes, net.num_zones, net.first_thru_node, precision, scenarios,
-                   device_name)).encode())
+                   device_name, "default")).encode())
     return h.hexdigest()
 
 
