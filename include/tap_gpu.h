@@ -239,12 +239,16 @@ typedef struct tapgpu_options_s {
                             (the queue kernels keep their bitmaps and ring in shared memory,
                             as they do whenever the labels do not fit); 2: all per-CTA
                             scratch in global memory */
-  int sssp_variant;      /* 0 default (6 up to 4096 nodes and links, else 4, or its 32-bit
-                            ring form above 65535 nodes); 1 bulk-synchronous
+  int sssp_variant;      /* 0 default (6 up to 4096 nodes and links; FP64 iterations and
+                            loadings above on the elimination hierarchy where it pays,
+                            unless an option from sssp_block on asks for something else;
+                            else 4, or its 32-bit ring form above 65535 nodes);
+                            1 bulk-synchronous
                             rounds; 2 asynchronous warp-owned frontier; 3 asynchronous near
                             set below a rising threshold; 4 as 3 with a FIFO ring of near
                             nodes (networks of at most 65535 nodes); 6 Bellman-Ford
-                            sweeps over the edge list held in shared memory (the default
+                            sweeps over the edge list, held in registers or, with a
+                            block size of the caller's, in shared memory (the default
                             for networks of at most 4096 nodes and 4096 links) */
   double nf_delta;       /* threshold step of variants 3 and 4 in cost units; 0 = 16 x mean
                             link cost */
@@ -274,6 +278,8 @@ const char *tapgpu_status_string(int status);
 /* message of the last failing call on this thread */
 const char *tapgpu_last_message(void);
 
+/* A context that may take the elimination hierarchy makes its plan in a thread of
+ * its own from here on; the first solve or loading waits for it. */
 int tapgpu_create(const tapgpu_network *net, const tapgpu_demand *dem,
                   const tapgpu_options *opt, tapgpu_ctx **out);
 void tapgpu_destroy(tapgpu_ctx *ctx);
@@ -303,7 +309,11 @@ int tapgpu_set_capacity(tapgpu_ctx *ctx, const double *capacity);
  * scen_links[scen_ptr[s] .. scen_ptr[s+1]-1] by scen_cap[...].  All scenarios
  * share topology and demand and are solved together on the device.
  * x0: optional warm-start volumes [M] applied to every scenario.
- * results: [num_scen]. */
+ * results: [num_scen].
+ * FP64: the number of scenarios decides, with the network's size, whether the
+ * iterations run on the elimination hierarchy.  Where paths cost exactly the same,
+ * it may load another of them than label correction, so a scenario's flows can
+ * then differ between a small batch and a large one. */
 int tapgpu_solve_scenarios(tapgpu_ctx *ctx, int num_scen, const int64_t *scen_ptr,
                            const int64_t *scen_links, const double *scen_cap, int max_iters,
                            double target_relgap, const double *x0, tapgpu_result *results);
@@ -328,7 +338,8 @@ int tapgpu_profile_iteration(tapgpu_ctx *ctx, int reps, float *ms);
 
 /* Run `iters` further FW iterations of every scenario of the last solve
  * (ignoring the stopping rule), without host synchronisation in between
- * unless kernel timing is on. */
+ * unless kernel timing is on.  On the elimination hierarchy the call waits for
+ * the last of them. */
 int tapgpu_run_iterations(tapgpu_ctx *ctx, int iters);
 
 /* Kernel timing: with `on`, CUDA events are recorded around every launch of

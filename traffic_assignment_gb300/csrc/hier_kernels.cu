@@ -31,15 +31,16 @@
 // up to 2^-53 of the sum at every link.
 //
 // One iteration of 10,000 nodes and 1,000 origins (220,000 arcs, 14 million
-// relaxations): label correction and tree walks 1.70 ms for one scenario, 22.2
-// ms for 16; the hierarchy 1.31 and 5.7 ms.  By kernel, us for 1 and 16
-// scenarios: weights 5 / 39, bottom 34 / 82, tiles 36 x 10 / 36 x 17, mark 46 /
-// 377, mark_far 6 / 39, climb 200 / 1100, top 248 / 1515, subs 84 / 1090,
-// volumes 153 / 415, descend 74 / 204, collect 4 / 35, passes 12 x 12 / 12 x
-// 30, links 4 / 12.  With one scenario every kernel is bound by its chain of
-// dependent steps (levels, chunks of an origin's path, rows of a subtree), so
-// they are cut to keep the chain short; with many by the 64-bit additions and
-// comparisons of the climb and the sweep.
+// relaxations): label correction and tree walks 1.67 ms for one scenario, 21.9
+// ms for 16; the hierarchy 1.33 and 5.99 ms.  By kernel, us for 1 and 16
+// scenarios: weights 6 / 42, bottom 35 / 82, tiles 38 x 8 / 38 x 16 (from one's end
+// to the next one's), mark 46 / 377, mark_far 6 / 35, climb 200 / 1100, top 248 /
+// 1520, subs 85 / 1124, volumes 153 / 453, descend 75 / 210, collect 4 / 35,
+// passes 12 x 12 / 12 x 32, split 8 / 15, links 5 / 13, exponents 2 / 2.  With one
+// scenario every kernel is bound by its chain of dependent steps (levels, chunks
+// of an origin's path, rows of a subtree), so they are cut to keep the chain
+// short; with many by the 64-bit additions and comparisons of the climb and the
+// sweep.
 #include "hier_kernels.cuh"
 
 #include <cooperative_groups.h>
@@ -1410,7 +1411,10 @@ __global__ void __launch_bounds__(kElimBlock) k_hier_collect(HierArgs a) {
 }
 
 constexpr int kSplitBlock = 256;
-constexpr int kSplitPasses = 12;  // launched with the whole grid
+// Passes launched with the whole grid.  What they leave takes the one block of
+// k_hier_split 8 us at 10,000 nodes, 15 at 40,000 and 24 at 100,000, of 1.3, 3.4
+// and 7.4 ms an iteration (4 scenarios of 40,000 nodes 15, 2 of 100,000 27).
+constexpr int kSplitPasses = 12;
 
 // One pass over a scenario's listed shortcuts: a shortcut's volume passes to
 // the two arcs of its split.  The first goes on in the same thread at once,

@@ -336,10 +336,14 @@ int Ctx::alloc_scenarios(int S) {
 //     there is to do; 3.5 per 10^6 relaxations of an elimination per
 //     scenario; 1.2 per 10^6 arcs and origin
 // Measured, hierarchy : label correction in ms: 10,000 nodes, 1,000 origins, 1
-// scenario 1.34 : 1.70, 4 scenarios 2.31 : 5.77, 16 scenarios 6.04 : 22.2; 40
-// origins, 64 scenarios 5.42 : 3.66; 3,569 nodes, 101 origins, 16 scenarios
-// 1.08 : 0.93, 64 scenarios 1.93 : 3.14; 22,500 nodes, 400 origins, 1 scenario
-// 2.02 : 1.86, 2 scenarios 2.24 : 3.55.
+// scenario 1.33 : 1.67, 4 scenarios 2.30 : 5.70, 16 scenarios 5.99 : 21.9; 40
+// origins, 64 scenarios 5.42 : 3.63; 3,569 nodes, 101 origins, 16 scenarios
+// 0.87 : 0.92, 64 scenarios 1.76 : 3.10; 22,500 nodes, 400 origins, 1 scenario
+// 1.83 : 1.83, 2 scenarios 2.06 : 3.47; 40,000 nodes, 1,000 origins, 1 scenario
+// 3.41 : 8.27, 4 scenarios 7.38 : 25.0.  Above the fitted sizes the line lies on
+// the safe side: 60,000 nodes, 500 origins, 1 scenario 4.45 : 6.86, 4 scenarios
+// 7.78 : 20.4; 100,000 nodes, 1,000 origins, 1 scenario 7.39 : 21.7, 4 scenarios
+// 21.3 : 69.2, where the fits give 10.3 : 19.2 and 31.9 : 58.9.
 bool Ctx::hier_pays(int nscen, int levels, double relaxations, int arcs) const {
   const double kn = n1 * 1e-3, tasks = static_cast<double>(nscen) * Z;
   const double one = sssp_smem ? std::min(100.0 + 27.0 * kn, 250.0 + 15.5 * kn) : 80.0 * kn;
